@@ -993,7 +993,7 @@ int32_t close_block(vn_model* m, GemmArgs g, const float* bias, const Next& next
 int32_t batched(vn_model* m, const GemmArgs& g) {
   if (m->cfg.bf16 && gemm_mma_supported(g)) return launch_gemm_mma(m->ctx, g);
   if (m->cfg.bf16) return launch_gemm_simt<__nv_bfloat16, __nv_bfloat16>(m->ctx, g);
-  return launch_gemm_simt<float, float>(m->ctx, g);
+  return launch_gemm_f32(m->ctx, g);
 }
 
 // ---- mixers: normalised rows -> the input of the output projection -----------------------------------------------------------

@@ -3,6 +3,7 @@
 // TriSparseAttention.forward accepts (tri_sparse_attn.py:559-575) kept resident and updated in place.
 #include "common.cuh"
 #include "gemm.cuh"
+#include "gemm_f32.cuh"
 #include "gemm_mma.cuh"
 #include "model_kernels.cuh"
 #include "attn_mma.cuh"
@@ -408,7 +409,7 @@ int32_t linear(vn_model* m, GemmArgs g) {
     if (gemm_mma_supported(g)) return launch_gemm_mma(ctx, g);
     return launch_gemm_simt<__nv_bfloat16, __nv_bfloat16>(ctx, g);
   }
-  return launch_gemm_simt<float, float>(ctx, g);
+  return launch_gemm_f32(ctx, g);
 }
 
 // The attention part of a vda / dsa / kda / gmla layer (verse_nex/delta_attention.py): m->h (normalised rows) ->
@@ -1206,7 +1207,7 @@ int32_t compute_sinks(vn_model* m, int mode) {
         }
         g.W = (char*)S.wqkv + (size_t)(qd + which * kvd) * D * m->esz;
         if (c.bf16) TRY((launch_gemm_simt<__nv_bfloat16, __nv_bfloat16>(ctx, g)));
-        else TRY((launch_gemm_simt<float, float>(ctx, g)));
+        else TRY(launch_gemm_f32(ctx, g));
       }
     }
     if (is_delta(L.kind)) continue;
@@ -1224,7 +1225,7 @@ int32_t compute_sinks(vn_model* m, int mode) {
       } else {
         g.W = (char*)L.wqkv + (size_t)(qd + which * kvd) * D * m->esz;
         if (c.bf16) TRY((launch_gemm_simt<__nv_bfloat16, __nv_bfloat16>(ctx, g)));
-        else TRY((launch_gemm_simt<float, float>(ctx, g)));
+        else TRY(launch_gemm_f32(ctx, g));
       }
     }
   }

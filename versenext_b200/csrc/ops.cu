@@ -1,11 +1,13 @@
 // DeviceBackend operator set in fp32 (verse_torch/device.py:219-270; NumPy semantics of :285-335).
 #include "common.cuh"
 #include "gemm.cuh"
+#include "gemm_f32.cuh"
 #include <math_constants.h>
 #include <stdint.h>
 #include <stdlib.h>
 
 namespace {
+using namespace f32_detail;
 
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
@@ -82,94 +84,242 @@ __global__ void rope_kernel(const float* __restrict__ x, const float* __restrict
   y[row * D + half + j] = x1 * s + x2 * c;
 }
 
-// one warp per query row: scores over Tk keys, softmax, weighted sum of V
-__global__ void __launch_bounds__(128) attention_kernel(const float* __restrict__ q, const float* __restrict__ k,
-                                                        const float* __restrict__ v, const float* __restrict__ mask,
-                                                        float* __restrict__ out, long long Tq, long long Tk, int D,
-                                                        float scale) {
-  extern __shared__ float smem[];  // 4 warps x Tk scores
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long qi = (long long)blockIdx.x * 4 + warp;
-  const long long bh = blockIdx.y;
-  if (qi >= Tq) return;
-  float* sc = smem + (long long)warp * Tk;
+// ---- attention over fp32 heads ------------------------------------------------------------------------------------------
+// four values of a row from element d on; elements from D on are zero
+__device__ __forceinline__ float4 row4(const float* __restrict__ r, int d, int D, bool vec) {
+  if (vec) return d < D ? *reinterpret_cast<const float4*>(r + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+  return make_float4(d < D ? r[d] : 0.f, d + 1 < D ? r[d + 1] : 0.f, d + 2 < D ? r[d + 2] : 0.f, d + 3 < D ? r[d + 3] : 0.f);
+}
+
+// Few queries, or heads too wide for the tile kernel: a block per query row, any D.  `lpk` lanes (a power of two) share a key's
+// dot product in float4 steps, so that a warp reads whole rows; scores stay in shared memory; for the values `lpk` threads
+// cover a row and the block's groups of them take every (256 / lpk)-th key, summed at the end.
+__global__ void __launch_bounds__(256) attention_row_kernel(const float* __restrict__ q, const float* __restrict__ k,
+                                                            const float* __restrict__ v, const float* __restrict__ mask,
+                                                            float* __restrict__ out, long long Tq, int Tk, int D, float scale,
+                                                            int lpk, int vec) {
+  extern __shared__ __align__(16) float smem[];      // Tk scores, then 256 partial float4
+  __shared__ float red[8];
+  float* sc = smem;
+  float4* part = reinterpret_cast<float4*>(smem + ((Tk + 3) & ~3));
+  const int tid = threadIdx.x;
+  const long long qi = blockIdx.x, bh = blockIdx.y;
   const float* qr = q + (bh * Tq + qi) * D;
   const float* kb = k + bh * Tk * D;
   const float* vb = v + bh * Tk * D;
+  const int grp = tid / lpk, li = tid % lpk, ng = 256 / lpk;
   float m = -CUDART_INF_F;
-  for (long long j = lane; j < Tk; j += 32) {
+  for (int j0 = 0; j0 < Tk; j0 += ng) {              // all lanes of a warp take the same trips
+    const int j = j0 + grp;
     float s = 0.f;
-    for (int d = 0; d < D; ++d) s = fmaf(qr[d], kb[j * D + d], s);
-    s *= scale;
-    if (mask) s += mask[qi * Tk + j];
-    sc[j] = s;
-    m = fmaxf(m, s);
+    if (j < Tk)
+      for (int d = li * 4; d < D; d += lpk * 4) {
+        const float4 a = row4(qr, d, D, vec), b = row4(kb + (long long)j * D, d, D, vec);
+        s = fmaf(a.x, b.x, s); s = fmaf(a.y, b.y, s); s = fmaf(a.z, b.z, s); s = fmaf(a.w, b.w, s);
+      }
+    for (int o = lpk >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (j < Tk) {
+      s *= scale;
+      if (mask) s += mask[qi * Tk + j];
+      if (li == 0) sc[j] = s;
+      m = fmaxf(m, s);
+    }
   }
-  m = warp_max(m);
+  m = block_reduce<256>(m, true, red);               // its barriers also publish the scores
   float l = 0.f;
-  for (long long j = lane; j < Tk; j += 32) { float e = expf(sc[j] - m); sc[j] = e; l += e; }
-  l = warp_sumf(l);
-  __syncwarp();
-  for (int d = lane; d < D; d += 32) {
-    float acc = 0.f;
-    for (long long j = 0; j < Tk; ++j) acc = fmaf(sc[j] / l, vb[j * D + d], acc);
-    out[(bh * Tq + qi) * D + d] = acc;
+  for (int j = tid; j < Tk; j += 256) { const float e = expf(sc[j] - m); sc[j] = e; l += e; }
+  l = block_reduce<256>(l, false, red);
+  __syncthreads();
+  for (int d0 = 0; d0 < D; d0 += lpk * 4) {
+    const int d = d0 + li * 4;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (d < D)
+      for (int j = grp; j < Tk; j += ng) {
+        const float p = sc[j];
+        const float4 x = row4(vb + (long long)j * D, d, D, vec);
+        acc.x = fmaf(p, x.x, acc.x); acc.y = fmaf(p, x.y, acc.y); acc.z = fmaf(p, x.z, acc.z); acc.w = fmaf(p, x.w, acc.w);
+      }
+    part[tid] = acc;
+    __syncthreads();
+    for (int e = tid; e < lpk * 4; e += 256) {
+      if (d0 + e < D) {
+        float s = 0.f;
+        for (int gi = 0; gi < ng; ++gi) s += reinterpret_cast<const float*>(part)[gi * lpk * 4 + e];
+        out[(bh * Tq + qi) * D + d0 + e] = s / l;
+      }
+    }
+    __syncthreads();
   }
 }
 
-
-// ---- fp32 linear for a few rows against a large weight matrix (the k draft heads of SpeculativeDecoder.draft:
-// 4 x 248,320 x 1,024 fp32 = 4 GB of weights for 1 to 32 hidden rows, speculative.py:150-158) -------------------
-// Weight streaming: a warp owns SK_NR consecutive output features and walks K in float4 steps, one 512-byte coalesced
-// segment of every weight row per trip, against up to 8 rows of x at a time (x is a few KB: it stays in L1).  With
-// more than 8 rows the warp makes one pass per group of 8 over the same weight rows, which it finds in L1 / L2, so
-// DRAM still sees every weight once.  Per output: each lane sums its k = 4 * lane + 128 * i terms in order, then the
-// lanes are added by a shuffle tree: deterministic.
-constexpr int SK_NR = 4;
-template <int MR>
-__global__ void __launch_bounds__(256, 2) linear_skinny_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                            const float* __restrict__ bias, float* __restrict__ y,
-                                                            int M, long long N, int K) {
-  const int lane = threadIdx.x & 31;
-  const long long n0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * SK_NR;
-  if (n0 >= N) return;
-  const float* wr[SK_NR];
+// Tiles of 64 queries x 64 keys, heads of up to DM.  A warp owns 16 query rows; its 16 lanes of a row hold the row's scores of four
+// keys each, so that the online soft-max needs shuffles only, and DM / 16 of its results.  Per thread 8 x 4 products of
+// float4s along the head (12 shared loads for 128 FMAs) for the scores, 8 x DM / 16 along the keys for the values: the
+// bound is the FMA rate over those loads.  The next keys arrive while values are summed and the values while scores are.
+constexpr int AT_Q = 64, AT_K = 64;
+template <int DM>
+struct AttnTile {
+  static constexpr int LD = DM + 4, LDP = AT_K + 4;
+  static constexpr size_t SMEM = (size_t)(3 * AT_Q * LD + AT_Q * LDP) * sizeof(float);
+};
+template <int DM>
+__global__ void __launch_bounds__(128) attention_tile_kernel(const float* __restrict__ q, const float* __restrict__ k,
+                                                             const float* __restrict__ v, const float* __restrict__ mask,
+                                                             float* __restrict__ out, long long Tq, int Tk, int D, float scale,
+                                                             int vec) {
+  constexpr int LD = AttnTile<DM>::LD, LDP = AttnTile<DM>::LDP, DC = DM / 16;
+  extern __shared__ __align__(16) float smem[];
+  float* sQ = smem;
+  float* sK = sQ + AT_Q * LD;
+  float* sV = sK + AT_K * LD;
+  float* sP = sV + AT_K * LD;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ty = warp * 2 + (lane >> 4), tx = lane & 15;   // rows ty + 8 i, keys tx + 16 j
+  const long long bh = blockIdx.y, q0 = (long long)blockIdx.x * AT_Q;
+  const float* kb = k + bh * Tk * D;
+  const float* vb = v + bh * Tk * D;
+  // rows of a tile, zero beyond the last row and beyond D
+  auto load = [&](float* dst, const float* src, long long r0, long long rows) {
+    const unsigned base = (unsigned)__cvta_generic_to_shared(dst);
+    if (vec) {
+#pragma unroll 4
+      for (int e = tid; e < AT_K * (DM / 4); e += 128) {
+        const int r = e / (DM / 4), d = (e % (DM / 4)) * 4;
+        const bool ok = r0 + r < rows && d < D;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + (r * LD + d) * 4), "l"(src + (ok ? (r0 + r) * D + d : 0)), "r"(ok ? 16 : 0));
+      }
+    } else {
+#pragma unroll 4
+      for (int e = tid; e < AT_K * DM; e += 128) {
+        const int r = e / DM, d = e % DM;
+        const bool ok = r0 + r < rows && d < D;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(base + (r * LD + d) * 4), "l"(src + (ok ? (r0 + r) * D + d : 0)), "r"(ok ? 4 : 0));
+      }
+    }
+    asm volatile("cp.async.commit_group;");
+  };
+  load(sQ, q + bh * Tq * D, q0, Tq);
+  load(sK, kb, 0, Tk);
+  float m[8], l[8];
+  f32x2 o[8][DC / 2];
 #pragma unroll
-  for (int j = 0; j < SK_NR; ++j) wr[j] = w + (n0 + j < N ? n0 + j : N - 1) * (long long)K;
-  for (int m0 = 0; m0 < M; m0 += MR) {
-    float acc[SK_NR][MR];
+  for (int i = 0; i < 8; ++i) {
+    m[i] = -CUDART_INF_F; l[i] = 0.f;
 #pragma unroll
-    for (int j = 0; j < SK_NR; ++j)
+    for (int c = 0; c < DC / 2; ++c) o[i][c] = 0;
+  }
+  for (int k0 = 0; k0 < Tk; k0 += AT_K) {
+    load(sV, vb, k0, Tk);
+    asm volatile("cp.async.wait_group 1;");          // the keys (and the queries) are there
+    __syncthreads();
+    f32x2 s2[8][4];
 #pragma unroll
-      for (int i = 0; i < MR; ++i) acc[j][i] = 0.f;
-#pragma unroll 1
-    for (int k = lane * 4; k < K; k += 128) {
-      float4 wv[SK_NR];
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < SK_NR; ++j) wv[j] = *reinterpret_cast<const float4*>(wr[j] + k);
+      for (int j = 0; j < 4; ++j) s2[i][j] = 0;
+#pragma unroll 2
+    for (int d = 0; d < DM; d += 4) {
+      ulonglong2 a[8];
 #pragma unroll
-      for (int i = 0; i < MR; ++i) {
-        const int m = m0 + i < M ? m0 + i : M - 1;
-        const float4 xv = __ldg(reinterpret_cast<const float4*>(x + (long long)m * K + k));
+      for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(sQ + (ty + 8 * i) * LD + d);
 #pragma unroll
-        for (int j = 0; j < SK_NR; ++j) {
-          acc[j][i] = fmaf(xv.x, wv[j].x, acc[j][i]);
-          acc[j][i] = fmaf(xv.y, wv[j].y, acc[j][i]);
-          acc[j][i] = fmaf(xv.z, wv[j].z, acc[j][i]);
-          acc[j][i] = fmaf(xv.w, wv[j].w, acc[j][i]);
+      for (int j = 0; j < 4; ++j) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(sK + (tx + 16 * j) * LD + d);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          fma2(s2[i][j], a[i].x, b.x);
+          fma2(s2[i][j], a[i].y, b.y);
         }
       }
     }
 #pragma unroll
-    for (int j = 0; j < SK_NR; ++j)
+    for (int i = 0; i < 8; ++i) {
+      const long long row = q0 + ty + 8 * i;
+      float top = m[i], s[4];
 #pragma unroll
-      for (int i = 0; i < MR; ++i) {
-        float v = acc[j][i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0 && m0 + i < M && n0 + j < N) y[(long long)(m0 + i) * N + n0 + j] = v + (bias ? bias[n0 + j] : 0.f);
+      for (int j = 0; j < 4; ++j) {
+        const int key = k0 + tx + 16 * j;
+        s[j] = sum2(s2[i][j]) * scale;
+        if (mask && row < Tq && key < Tk) s[j] += mask[row * Tk + key];
+        if (key >= Tk) s[j] = -CUDART_INF_F;
+        top = fmaxf(top, s[j]);
       }
+#pragma unroll
+      for (int x = 8; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
+      // nothing but -inf so far: exponentials of -inf are then zero, and a row of nothing else ends as 0 / 0
+      const float at = top == -CUDART_INF_F ? 0.f : top;
+      const float fade = expf(m[i] - at);
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float e = expf(s[j] - at);
+        sP[(ty + 8 * i) * LDP + tx + 16 * j] = e;
+        sum += e;
+      }
+#pragma unroll
+      for (int x = 8; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
+      l[i] = l[i] * fade + sum;
+      m[i] = top;
+#pragma unroll
+      for (int c = 0; c < DC / 2; ++c) {
+        const float2 t = unpack2(o[i][c]);
+        o[i][c] = pack2(t.x * fade, t.y * fade);
+      }
+    }
+    asm volatile("cp.async.wait_group 0;");          // the values are there
+    __syncthreads();                                 // and the keys' tile is free
+    if (k0 + AT_K < Tk) load(sK, kb, k0 + AT_K, Tk);
+    else asm volatile("cp.async.commit_group;");
+#pragma unroll 2
+    for (int j = 0; j < AT_K; j += 4) {
+      float4 p[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) p[i] = *reinterpret_cast<const float4*>(sP + (ty + 8 * i) * LDP + j);
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        f32x2 x[DC / 2];
+#pragma unroll
+        for (int c = 0; c < DC / 2; c += (DC < 4 ? 1 : 2)) {
+          if (DC < 4) {
+            x[c] = *reinterpret_cast<const f32x2*>(sV + (j + jj) * LD + tx * 2);
+          } else {
+            const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(sV + (j + jj) * LD + tx * 4 + c * 32);
+            x[c] = t.x; x[(c + 1) % (DC / 2)] = t.y;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float w = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
+          const f32x2 ww = pack2(w, w);
+#pragma unroll
+          for (int c = 0; c < DC / 2; ++c) fma2(o[i][c], ww, x[c]);
+        }
+      }
+    }
+    __syncthreads();                                 // the values' tile is free
   }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const long long row = q0 + ty + 8 * i;
+    if (row >= Tq) continue;
+#pragma unroll
+    for (int c = 0; c < DC / 2; ++c) {
+      const int d = DC < 4 ? tx * 2 : tx * 4 + (c >> 1) * 64 + (c & 1) * 2;
+      const float2 t = unpack2(o[i][c]);
+      if (d < D) out[(bh * Tq + row) * D + d] = t.x / l[i];
+      if (d + 1 < D) out[(bh * Tq + row) * D + d + 1] = t.y / l[i];
+    }
+  }
+}
+
+template <int DM>
+int32_t launch_attention_tile(vn_ctx* ctx, const float* q, const float* k, const float* v, const float* mask, float* out, int64_t BH,
+                              int64_t Tq, int64_t Tk, int D, float scale, int vec) {
+  constexpr size_t smem = AttnTile<DM>::SMEM;
+  VN_CUDA(ctx, cudaFuncSetAttribute(attention_tile_kernel<DM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  dim3 grid((unsigned)ceil_div(Tq, (int64_t)AT_Q), (unsigned)BH);
+  VN_LAUNCH(ctx, attention_tile_kernel<DM>, grid, 128, smem, q, k, v, mask, out, (long long)Tq, (int)Tk, D, scale, vec);
+  return VN_OK;
 }
 
 }  // namespace
@@ -187,7 +337,7 @@ int32_t vn_matmul(vn_ctx* ctx, const float* a, const float* b, float* c, int64_t
   g.W = b; g.ldw = 1; g.ldw_k = N; g.w_stride = b_broadcast ? 0 : K * N;
   g.C = c; g.ldc = N; g.c_stride = M * N;
   g.M = (int)M; g.N = (int)N; g.K = (int)K; g.nseg = (int)batch;
-  return launch_gemm_simt<float, float>(ctx, g);
+  return launch_gemm_f32(ctx, g);
 }
 
 int32_t vn_linear(vn_ctx* ctx, const float* x, const float* w, const float* bias, float* y, int64_t M, int64_t N,
@@ -196,21 +346,10 @@ int32_t vn_linear(vn_ctx* ctx, const float* x, const float* w, const float* bias
   VN_REQUIRE(ctx, x && w && y, "null pointer");
   VN_REQUIRE(ctx, M >= 0 && N >= 0 && K >= 0, "bad shape");
   if (M * N == 0) return VN_OK;
-  // few rows against many output features: the weight-streaming kernel
-  // VN_LINEAR_SKINNY_MAX: most rows the streaming kernel takes (default 32; 0 keeps the tiled kernel: A/B timing)
-  static const int skinny_max = [] { const char* e = getenv("VN_LINEAR_SKINNY_MAX"); return e ? atoi(e) : 32; }();
-  if (M <= skinny_max && N >= 1024 && K % 4 == 0 && K >= 128 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
-    const unsigned grid = (unsigned)ceil_div(N, (int64_t)(8 * SK_NR));
-    if (M == 1) VN_LAUNCH(ctx, linear_skinny_kernel<1>, grid, 256, 0, x, w, bias, y, (int)M, (long long)N, (int)K);
-    else if (M == 2) VN_LAUNCH(ctx, linear_skinny_kernel<2>, grid, 256, 0, x, w, bias, y, (int)M, (long long)N, (int)K);
-    else if (M <= 4) VN_LAUNCH(ctx, linear_skinny_kernel<4>, grid, 256, 0, x, w, bias, y, (int)M, (long long)N, (int)K);
-    else VN_LAUNCH(ctx, linear_skinny_kernel<8>, grid, 256, 0, x, w, bias, y, (int)M, (long long)N, (int)K);
-    return VN_OK;
-  }
   GemmArgs g;
   g.A = x; g.lda = K; g.W = w; g.ldw = K; g.C = y; g.ldc = N; g.bias = bias;
   g.M = (int)M; g.N = (int)N; g.K = (int)K;
-  return launch_gemm_simt<float, float>(ctx, g);
+  return launch_gemm_f32(ctx, g);
 }
 
 int32_t vn_softmax(vn_ctx* ctx, const float* x, float* y, int64_t outer, int64_t n, int64_t inner) {
@@ -256,13 +395,23 @@ int32_t vn_attention(vn_ctx* ctx, const float* q, const float* k, const float* v
   VN_REQUIRE(ctx, q && k && v && out && BH >= 0 && Tq >= 0 && Tk >= 1 && D >= 1, "bad arguments");
   VN_REQUIRE(ctx, BH < 65536, "too many batch*heads");
   if (BH * Tq == 0) return VN_OK;
-  const size_t smem = (size_t)4 * Tk * sizeof(float);
-  VN_REQUIRE(ctx, smem <= 200 * 1024, "Tk %lld too long for the backend attention op", (long long)Tk);
+  VN_REQUIRE(ctx, (size_t)4 * Tk * sizeof(float) <= 200 * 1024, "Tk %lld too long for the backend attention op", (long long)Tk);
+  const int vec = D % 4 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0;
+  const float scale = 1.0f / sqrtf((float)D);
+  // A tile's 64 rows share the keys that are loaded; below a quarter of them a block per row is as fast and spreads over more SMs.
+  if (Tq >= 16 && D <= 128) {
+    if (D <= 32) return launch_attention_tile<32>(ctx, q, k, v, mask, out, BH, Tq, Tk, (int)D, scale, vec);
+    if (D <= 64) return launch_attention_tile<64>(ctx, q, k, v, mask, out, BH, Tq, Tk, (int)D, scale, vec);
+    return launch_attention_tile<128>(ctx, q, k, v, mask, out, BH, Tq, Tk, (int)D, scale, vec);
+  }
+  int lpk = 1;
+  while (lpk < 32 && lpk * 4 < D) lpk *= 2;
+  const size_t smem = (size_t)((Tk + 3) & ~(int64_t)3) * sizeof(float) + 256 * sizeof(float4);
   if (smem > 48 * 1024)
-    VN_CUDA(ctx, cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((unsigned)ceil_div(Tq, (int64_t)4), (unsigned)BH);
-  VN_LAUNCH(ctx, attention_kernel, grid, 128, smem, q, k, v, mask, out, (long long)Tq, (long long)Tk, (int)D,
-            1.0f / sqrtf((float)D));
+    VN_CUDA(ctx, cudaFuncSetAttribute(attention_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  VN_REQUIRE(ctx, Tq < (1ll << 31), "too many queries");
+  dim3 grid((unsigned)Tq, (unsigned)BH);
+  VN_LAUNCH(ctx, attention_row_kernel, grid, 256, smem, q, k, v, mask, out, (long long)Tq, (int)Tk, (int)D, scale, lpk, vec);
   return VN_OK;
 }
 
