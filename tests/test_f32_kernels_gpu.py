@@ -49,3 +49,30 @@ def test_attention(BH, Tq, Tk, D, masked):
         assert np.all(np.isnan(got[:, -1])) and np.all(np.isnan(want[:, -1]))
         got, want = got[:, :-1], want[:, :-1]
     assert np.all(np.abs(got - want) <= (2 * err + (Tk + 8) * EPS) * np.abs(v).max())
+
+
+@pytest.mark.parametrize("n_head,n_kv,dim,window,n_sink,alibi,ctx,new,tree", [
+    (4, 4, 64, 32, 4, True, 40, 5, False), (4, 2, 96, 16, 3, True, 0, 70, False), (2, 1, 128, 24, 1, False, 70, 1, False), (4, 1, 160, 64, 65, True, 61, 17, False),
+    (8, 2, 64, 1100, 2, True, 1020, 3, False), (8, 2, 64, 100, 2, True, 1023, 3, False), (4, 2, 256, 20, 7, True, 30, 9, True), (2, 2, 32, 8, 1, False, 0, 400, False)])
+def test_three_path_attention(n_head, n_kv, dim, window, n_sink, alibi, ctx, new, tree):
+    """Rows of the float32 model's attention at the edges of its blocks (rows that do not fill one, groups of query heads,
+    contexts around a key tile, the window, ALiBi's switch, more blocks than SMs) against the restated forward."""
+    from oracle import model as OM
+    cfg = OM.small_config(vocab_size=50, dim=dim, n_layer=1, n_head=n_head, n_kv_head=n_kv, window_size=window, num_global_tokens=n_sink,
+                          use_alibi=alibi, use_rope=not alibi, max_seq_len=2048, init_std=0.2)
+    sd = OM.init_state_dict(cfg, seed=5, gate_std=1.0)
+    kw = cfg.to_dict()
+    kw.pop("init_std")
+    m = vn.VerseNexLM(dtype="f32", **kw)
+    m.load_state_dict(sd)
+    B = 40 if new >= 400 else 2
+    toks = np.random.default_rng(1).integers(0, 50, (B, ctx + new))
+    parents = [-1, -1, 0, 0, 1, 2, 2, 5, 4][:new] if tree else None
+    cache, oc = m.new_cache(B, ctx + new + 1), None
+    if ctx:
+        m.forward_cached(toks[:, :ctx], cache, last_only=True)
+        cache.commit(ctx, np.full(B, ctx, np.int32))
+        _, oc = OM.forward(sd, cfg, toks[:, :ctx])
+    got = m.forward_cached(toks[:, ctx:], cache, parents=parents).numpy()
+    want, _ = OM.forward(sd, cfg, toks[:, ctx:], cache=oc, parents=parents)
+    assert np.max(np.abs(got - want)) / np.max(np.abs(want)) < 1e-4      # float32 on both sides, sums in other orders

@@ -554,8 +554,7 @@ int32_t forward_t(vn_model* m, vn_kv* kv, const int64_t* tokens, int B, int Tn, 
     } else if (attn_mma_supported(a, c.bf16 != 0) && !m->force_simt_attn) {
       TRY(launch_attn_mma(ctx, a, B));
     } else {
-      dim3 grid(ceil_div(H, 8), M);
-      VN_LAUNCH(ctx, trisparse_attn_kernel<T>, grid, 256, 0, a);
+      TRY(launch_trisparse<T>(ctx, a, B));
     }
     }
     g = GemmArgs();
@@ -962,8 +961,7 @@ int32_t forward_tc(vn_model* m, vn_kv* kv, const int64_t* tokens, int B, int Tn,
     if (attn_tc) {
       TRY(launch_attn_mma(ctx, a, B));
     } else {
-      dim3 grid(ceil_div(H, 8), M);
-      VN_LAUNCH(ctx, trisparse_attn_kernel<T>, grid, 256, 0, a);
+      TRY(launch_trisparse<T>(ctx, a, B));
     }
     }
     g = GemmArgs();

@@ -376,6 +376,195 @@ __global__ void __launch_bounds__(256) trisparse_attn_kernel(AttnArgs a) {
   }
 }
 
+// The same attention for a block of R query rows of one (sequence, key head), R consecutive (position, head of the group) pairs:
+// the three paths share one product with the keys and one with the values.  (1) scores of every key a row of the block may see
+// and of the sinks, key tiles of 64 through shared memory, into S[R][total]; (2) a warp per row: the three soft-maxes' sums, then
+// each score is replaced by the sum of its gated probabilities; (3) S times the values, tile by tile.  Bound by latency: small
+// models have few rows and a warp that walks the keys alone (the kernel above) spends its time in a chain of exponentials,
+// 8 to 20 us a layer where this one takes 4 to 9 (float32, 64 wide heads, 5 rows at context 32, 2 x 300 rows of prompts).
+constexpr int TR_TILE = 64, TR_THREADS = 128;
+template <typename T, int R>
+__global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, int cap) {
+  extern __shared__ __align__(16) float tr_smem[];
+  const int hd = a.hd, nq = hd >> 2, ld = hd + 4;
+  float* sT = tr_smem;                     // [TR_TILE][ld] a tile of keys or values
+  float* sQ = sT + TR_TILE * ld;           // [R][hd]
+  float* S = sQ + R * hd;                  // [R][cap]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n_rep = a.H / a.n_kv, n_items = a.Tn * n_rep;
+  const int i0 = blockIdx.x * R, kvh = blockIdx.y, b = blockIdx.z;
+  const int len = a.lens[b] + a.slot_offset;
+  const int t_first = i0 / n_rep, t_last = min(i0 + R - 1, n_items - 1) / n_rep;
+  const int span = max(a.window, a.alibi_window);
+  const bool all = a.use_alibi && a.alibi_window == 0 && (a.anc ? len + 1 : len + a.Tn) <= a.alibi_max;   // path C sees every key
+  const int lo = all ? 0 : max(0, (a.anc ? len : len + t_first) - span + 1);
+  const int hi = min(a.anc ? len + a.Tn : len + t_last + 1, a.max_seq);
+  const int nk = max(0, min(hi - lo, cap - a.n_sink)), total = nk + a.n_sink;
+  const long long kstride = (long long)a.n_kv * hd, base = ((long long)b * a.max_seq * a.n_kv + kvh) * hd;
+
+  // a tile's rows: TR_TILE * nq float4s over the threads, at most 8 each (hd <= 64)
+  float4 pre[8];
+  auto fetch = [&](const void* cache, const void* sink, int j0) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int e = tid + u * TR_THREADS, r = e / nq, d = (e % nq) * 4, j = j0 + r;
+      pre[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < TR_TILE && j < total) {
+        const T* src = j < nk ? reinterpret_cast<const T*>(cache) + base + (long long)(lo + j) * kstride
+                              : reinterpret_cast<const T*>(sink) + (long long)(j - nk) * kstride + (long long)kvh * hd;
+        pre[u] = load4(src + d);
+      }
+    }
+  };
+  auto put = [&]() {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int e = tid + u * TR_THREADS, r = e / nq, d = (e % nq) * 4;
+      if (r < TR_TILE) *reinterpret_cast<float4*>(sT + r * ld + d) = pre[u];
+    }
+  };
+  fetch(a.kc, a.sink_k, 0);
+  for (int e = tid; e < R * nq; e += TR_THREADS) {
+    const int i = i0 + e / nq, d = (e % nq) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < n_items) v = *reinterpret_cast<const float4*>(a.q + (long long)(b * a.Tn + i / n_rep) * a.ld_q + (kvh * n_rep + i % n_rep) * hd + d);
+    *reinterpret_cast<float4*>(sQ + e * 4) = v;
+  }
+  // ---- scores: a thread has one key of the tile and half of the rows
+  for (int j0 = 0; j0 < total; j0 += TR_TILE) {
+    put();
+    __syncthreads();
+    if (j0 + TR_TILE < total) fetch(a.kc, a.sink_k, j0 + TR_TILE);
+    else fetch(a.vc, a.sink_v, 0);
+    const int r = tid & (TR_TILE - 1), h0 = (tid / TR_TILE) * (R / 2);
+    float s[R / 2];
+#pragma unroll
+    for (int i = 0; i < R / 2; ++i) s[i] = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < hd; d += 4) {
+      const float4 k = *reinterpret_cast<const float4*>(sT + r * ld + d);
+#pragma unroll
+      for (int i = 0; i < R / 2; ++i) {
+        const float4 q = *reinterpret_cast<const float4*>(sQ + (h0 + i) * hd + d);
+        s[i] = fmaf(q.x, k.x, s[i]); s[i] = fmaf(q.y, k.y, s[i]); s[i] = fmaf(q.z, k.z, s[i]); s[i] = fmaf(q.w, k.w, s[i]);
+      }
+    }
+    if (j0 + r < total)
+#pragma unroll
+      for (int i = 0; i < R / 2; ++i) S[(h0 + i) * cap + j0 + r] = s[i] * a.scale;
+    __syncthreads();
+  }
+  // ---- weights
+  for (int it = warp; it < R && i0 + it < n_items; it += TR_THREADS / 32) {
+    const int t = (i0 + it) / n_rep, h = kvh * n_rep + (i0 + it) % n_rep;
+    const int pos = len + (a.depth ? a.depth[t] : t);
+    const unsigned long long anc = a.anc ? a.anc[t] : 0ull;
+    int tk_eff = a.anc ? pos + 1 : len + a.Tn;
+    if (a.alibi_window > 0) tk_eff = min(pos + 1, a.alibi_window);
+    const bool use_c = a.use_alibi && tk_eff <= a.alibi_max;
+    const float slope = 1.0f / exp2f((float)(h + 1) / (float)a.H);
+    float* row = S + it * cap;
+    // distance of key j from the row's position where the row sees it, else -1
+    auto distance = [&](int j) {
+      const int slot = lo + j, n = slot - len;
+      if (n < 0) return pos - slot;
+      const bool vis = a.anc ? (anc >> n) & 1ull : n <= t;
+      return vis ? pos - (len + (a.depth ? a.depth[n] : n)) : -1;
+    };
+    float ma = -CUDART_INF_F, mb = ma, mc = ma, la = 0.f, lb = 0.f, lc = 0.f;
+    for (int j = lane; j < nk; j += 32) {
+      const int dist = distance(j);
+      if (dist < 0) continue;
+      if (dist < a.window) ma = fmaxf(ma, row[j]);
+      if (use_c && (a.alibi_window == 0 || dist < a.alibi_window)) mc = fmaxf(mc, row[j] - slope * (float)dist);
+    }
+    for (int j = nk + lane; j < total; j += 32) mb = fmaxf(mb, row[j]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      ma = fmaxf(ma, __shfl_xor_sync(0xffffffffu, ma, o));
+      mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+      mc = fmaxf(mc, __shfl_xor_sync(0xffffffffu, mc, o));
+    }
+    for (int j = lane; j < nk; j += 32) {
+      const int dist = distance(j);
+      if (dist < 0) continue;
+      if (dist < a.window) la += expf(row[j] - ma);
+      if (use_c && (a.alibi_window == 0 || dist < a.alibi_window)) lc += expf(row[j] - slope * (float)dist - mc);
+    }
+    for (int j = nk + lane; j < total; j += 32) lb += expf(row[j] - mb);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      la += __shfl_xor_sync(0xffffffffu, la, o);
+      lb += __shfl_xor_sync(0xffffffffu, lb, o);
+      lc += __shfl_xor_sync(0xffffffffu, lc, o);
+    }
+    const float ga = la > 0.f ? a.g_a / la : 0.f, gb = lb > 0.f ? a.g_b / lb : 0.f, gc = lc > 0.f ? a.g_c / lc : 0.f;
+    for (int j = lane; j < nk; j += 32) {
+      const int dist = distance(j);
+      float w = dist < 0 ? -1.f : 0.f;                   // below zero: not this row's key, whatever its value is
+      if (dist >= 0 && dist < a.window) w = ga * expf(row[j] - ma);
+      if (dist >= 0 && use_c && (a.alibi_window == 0 || dist < a.alibi_window)) w += gc * expf(row[j] - slope * (float)dist - mc);
+      row[j] = w;
+    }
+    for (int j = nk + lane; j < total; j += 32) row[j] = gb * expf(row[j] - mb);
+  }
+  // ---- values: a thread has four dims of one row, and where the block has threads for it every `slices`-th key
+  const int per = nq * R, slices = max(1, TR_THREADS / per), slice = tid / per, it = (tid % per) / nq, d = (tid % nq) * 4;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j0 = 0; j0 < total; j0 += TR_TILE) {
+    put();
+    __syncthreads();
+    if (j0 + TR_TILE < total) fetch(a.vc, a.sink_v, j0 + TR_TILE);
+    if (slice < slices) {
+      const int n = min(TR_TILE, total - j0);
+#pragma unroll 4
+      for (int r = slice; r < n; r += slices) {
+        const float w = S[it * cap + j0 + r];
+        const float4 v = *reinterpret_cast<const float4*>(sT + r * ld + d);
+        if (!(w < 0.f)) { acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w); }
+      }
+    }
+    __syncthreads();
+  }
+  if (slice < slices) *reinterpret_cast<float4*>(sT + slice * R * hd + it * hd + d) = acc;
+  __syncthreads();
+  for (int e = tid; e < R * hd; e += TR_THREADS) {
+    const int i = i0 + e / hd;
+    if (i >= n_items) continue;
+    float v = 0.f;
+    for (int z = 0; z < slices; ++z) v += sT[z * R * hd + e];
+    reinterpret_cast<T*>(a.out)[(long long)(b * a.Tn + i / n_rep) * a.H * hd + (kvh * n_rep + i % n_rep) * hd + e % hd] = from_f<T>(v);
+  }
+}
+
+// The rows kernel where a block's scores fit shared memory, else the one-warp-per-row kernel (windows of many thousand keys).
+template <typename T>
+inline int32_t launch_trisparse(vn_ctx* ctx, const AttnArgs& a, int B) {
+  const int n_rep = a.H / a.n_kv, n_items = a.Tn * n_rep;
+  // eight rows a block once that gives two blocks per SM, four (shorter soft-maxes per warp) before
+  const int R = (long long)ceil_div(n_items, 8) * a.n_kv * B >= 2ll * ctx->sm_count ? 8 : 4;
+  // keys a block may see: all of them while path C is on (at most alibi_max, and a tree's nodes), else a window
+  const long long grown = a.anc ? a.Tn : R;
+  long long keys = std::min<long long>(a.max_seq, (long long)std::max(a.window, a.alibi_window) + grown);
+  if (a.use_alibi && a.alibi_window == 0) keys = std::max(keys, std::min<long long>(a.max_seq, (long long)a.alibi_max + grown));
+  const long long cap = (keys + a.n_sink) | 1;
+  const long long smem = (TR_TILE * (a.hd + 4) + R * a.hd + R * cap) * 4;
+  if (smem > 160 * 1024 || B > 65535 || a.n_kv > 65535) {
+    dim3 grid(ceil_div(a.H, 8), B * a.Tn);
+    VN_LAUNCH(ctx, trisparse_attn_kernel<T>, grid, 256, 0, a);
+    return VN_OK;
+  }
+  dim3 grid(ceil_div(n_items, R), a.n_kv, B);
+  if (R == 8) {
+    if (smem > 48 * 1024) VN_CUDA(ctx, cudaFuncSetAttribute(trisparse_rows_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    VN_LAUNCH(ctx, (trisparse_rows_kernel<T, 8>), grid, TR_THREADS, smem, a, (int)cap);
+  } else {
+    if (smem > 48 * 1024) VN_CUDA(ctx, cudaFuncSetAttribute(trisparse_rows_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    VN_LAUNCH(ctx, (trisparse_rows_kernel<T, 4>), grid, TR_THREADS, smem, a, (int)cap);
+  }
+  return VN_OK;
+}
+
 // ---- MoD routing (mod.py:340-387, :748-770) ----------------------------------------------------------
 // One warp per token.  Part router: softmax over all P part logits.  Expert router of every part: top-k on the
 // logits (ties -> lower index first), softmax over the kept logits.  Slot s = p*top_k + j of a token holds
