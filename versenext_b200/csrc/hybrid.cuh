@@ -1352,7 +1352,7 @@ int32_t mixture(vn_model* m, const HLayer& L, int M, const Buffers& b, const Nex
   const float* sorted_w = scale ? b.sorted_w : nullptr;
   if (tc) {
     int *off = b.sub_seg, *cnt = off + b.sub_cap, *w = cnt + b.sub_cap;
-    VN_LAUNCH(ctx, mod_subseg_kernel, 1, 32, 0, (const int*)hm.exp_count, (const int*)hm.exp_off, mats, off, cnt, w, b.sub_cap);
+    VN_LAUNCH(ctx, mod_subseg_kernel, 1, 32, 0, (const int*)hm.exp_count, (const int*)hm.exp_off, mats, off, cnt, w, b.sub_cap, 256);
     VN_LAUNCH(ctx, gather_sorted_kernel<T>, M * S, 128, 0, (const T*)m->h, (const int*)b.sorted_row, (T*)b.hs, D, sorted_w);
     TRY(ensure_partial(m, 1024));
     for (GemmArgs* g : {&up, &down}) {

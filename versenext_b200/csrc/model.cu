@@ -12,6 +12,7 @@
 #include "gemm_tc.cuh"
 #include "gemm_mma_q.cuh"
 #include "gemm_tcq.cuh"
+#include "gemm_tcq_rows.cuh"
 #include "k1.h"
 
 #include <math.h>
@@ -355,7 +356,7 @@ int32_t ensure_rows(vn_model* m, int M) {
   // that a forward never allocates them: filled by kernels on the stream
   if (m->sub_seg) cudaFree(m->sub_seg);
   m->sub_seg = nullptr;
-  m->sub_cap = (int)(c.P * c.E + R * S / 256 + 2);
+  m->sub_cap = (int)(c.P * c.E + R * S / 128 + 2);
   TRY(dev_alloc(ctx, (void**)&m->sub_seg, (size_t)3 * m->sub_cap * sizeof(int)));
   if (has_mod) {
     TRY(dev_alloc(ctx, (void**)&m->y, R * S * D * 4));
@@ -384,6 +385,11 @@ int32_t ensure_partial(vn_model* m, size_t bytes);
 int32_t linear(vn_model* m, GemmArgs g) {
   vn_ctx* ctx = m->ctx;
   if (g.wq) {
+    // dense blocks: the tensor-core kernel (VN_GEMM_TCQ=0 keeps mma.sync)
+    if (m->use_tc && !g.seg_cnt && gemm_tcq_rows_supported(g) && g.M <= 65535 * 64) {
+      TRY(ensure_partial(m, 1024));                               // the error word
+      return launch_gemm_tcq_rows(ctx, g, g.M, m->tc_error);
+    }
     if (!gemm_mma_q_supported(g)) return vn_fail(ctx, VN_ERR_UNSUPPORTED, "quantised GEMM shape K=%d unsupported", g.K);
     return launch_gemm_mma_q(ctx, g);
   }
@@ -586,34 +592,39 @@ int32_t forward_t(vn_model* m, vn_kv* kv, const int64_t* tokens, int B, int Tn, 
       VN_LAUNCH(ctx, mod_offsets_kernel, 1, 32, 0, m->expert_count, m->expert_off, m->expert_cur, ne);
       VN_LAUNCH(ctx, mod_scatter_kernel, ceil_div(M * S, 256), 256, 0, m->slot_expert, m->expert_off, m->expert_cur,
                 m->sorted_row, m->slot_pos, M * S, S, (const float*)nullptr, (float*)nullptr);
-      // Many routed rows on a bf16 model: the experts' segments are cut into pieces of at most 256 rows and run on
-      // the tcgen05 kernel (rows copied into expert order first, so that TMA loads them; a piece names its expert's
+      // Many routed rows on a bf16 model: the experts' segments are cut into pieces of at most 256 rows (128 where the weights
+      // are quantised) and run on the tcgen05 kernels (rows copied into expert order first, so that TMA loads them; a piece names its expert's
       // weights through seg_w).  Otherwise the mma.sync kernels gather the rows themselves.
       const char* pe = getenv("VN_PREFILL_TC");
-      const int n_sub = ne + ceil_div(M * S, 256);
-      const bool tc_experts = std::is_same<T, __nv_bfloat16>::value && m->use_tc && !m->qmode && !(pe && pe[0] == '0') &&
+      const int piece = m->qmode ? tc_detail::QR_ROWS : 256;
+      const int n_sub = ne + ceil_div(M * S, piece);
+      const bool tc_experts = std::is_same<T, __nv_bfloat16>::value && m->use_tc && !(m->qmode && (D % 64 || eh % 64)) && !(pe && pe[0] == '0') &&
                               (long long)M * S > 256 && m->hs && D % 8 == 0 && eh % 8 == 0 && n_sub <= 65535 && n_sub <= m->sub_cap &&
                               tc_detail::encode_fn() != nullptr;
       if (tc_experts) {
         int* sub_off = m->sub_seg; int* sub_cnt = m->sub_seg + m->sub_cap; int* sub_w = m->sub_seg + 2 * m->sub_cap;
         VN_LAUNCH(ctx, mod_subseg_kernel, 1, 32, 0, (const int*)m->expert_count, (const int*)m->expert_off, ne, sub_off,
-                  sub_cnt, sub_w, n_sub);
+                  sub_cnt, sub_w, n_sub, piece);
         VN_LAUNCH(ctx, gather_sorted_kernel<T>, M * S, 128, 0, (const T*)m->h, (const int*)m->sorted_row, (T*)m->hs, D, (const float*)nullptr);
         TRY(ensure_partial(m, 1024));
         TcPlan plan;
         plan.error_flag = m->tc_error;
         g = GemmArgs();
         g.A = m->hs; g.lda = D; g.W = L.e_gateup; g.ldw = D; g.w_stride = (long long)2 * eh * D;
-        g.C = m->act; g.ldc = eh; g.M = 256; g.N = 2 * eh; g.K = D; g.epi = EPI_SWIGLU; g.c_bf16 = 1;
+        g.C = m->act; g.ldc = eh; g.M = piece; g.N = 2 * eh; g.K = D; g.epi = EPI_SWIGLU; g.c_bf16 = 1;
         g.seg_off = sub_off; g.seg_cnt = sub_cnt; g.seg_w = sub_w; g.n_w = ne; g.nseg = n_sub; g.tag = "gemm_expert_gateup";
-        TRY(launch_gemm_tc(ctx, g, (long long)M * S, plan));
+        pick(g, L.e_gateup, L.q[4], L.qs[4], 2 * eh);
+        if (g.wq) TRY(launch_gemm_tcq_rows(ctx, g, (long long)M * S, m->tc_error));
+        else TRY(launch_gemm_tc(ctx, g, (long long)M * S, plan));
         g = GemmArgs();
         g.A = m->act; g.lda = eh; g.W = L.e_down; g.ldw = eh; g.w_stride = (long long)D * eh; g.C = m->y; g.ldc = D;
-        g.M = 256; g.N = D; g.K = eh; g.seg_off = sub_off; g.seg_cnt = sub_cnt; g.seg_w = sub_w; g.n_w = ne; g.nseg = n_sub;
+        g.M = piece; g.N = D; g.K = eh; g.seg_off = sub_off; g.seg_cnt = sub_cnt; g.seg_w = sub_w; g.n_w = ne; g.nseg = n_sub;
         g.tag = "gemm_expert_down";
+        pick(g, L.e_down, L.q[5], L.qs[5], D);
         TcPlan plan2;
         plan2.error_flag = m->tc_error;
-        TRY(launch_gemm_tc(ctx, g, (long long)M * S, plan2));
+        if (g.wq) TRY(launch_gemm_tcq_rows(ctx, g, (long long)M * S, m->tc_error));
+        else TRY(launch_gemm_tc(ctx, g, (long long)M * S, plan2));
       } else {
       g = GemmArgs();
       g.A = m->h; g.lda = D; g.a_rows = m->sorted_row; g.W = L.e_gateup; g.ldw = D; g.w_stride = (long long)2 * eh * D;
