@@ -35,6 +35,9 @@ struct GemmArgs {
   int post = 0;                   // EPI_STORE: function of columns [0, post_n): 0 none, POST_SILU, POST_RELU2
   int post_n = 0;
   const void* mul = nullptr;      // EPI_STORE, plain and batched modes: factors of the results, laid out and typed as C
+  // rows of A are RMS-normalised first, x / sqrt(mean(x^2) + norm_eps) * norm (gemm_f32_norm_supported says where)
+  const float* norm = nullptr;
+  float norm_eps = 0.f;
   const char* tag = nullptr;      // name of the call site in the per-kernel timing report (string literal)
   // weight-only quantisation: W points at INT8 / packed INT4 bytes, ldw and w_stride stay in ELEMENTS
   int wq = 0;                     // 0 dense, 1 int8, 2 int4 per output row, 3 int4 with one scale per 128 inputs

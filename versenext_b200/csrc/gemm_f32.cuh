@@ -159,14 +159,35 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_f32_kernel(G
 // pass per group of MR over the same weight rows, which it finds in L1 / L2, so DRAM still sees every weight once.  Per
 // output each lane sums its k = 4 lane + 128 i terms in order (even and odd apart), then the lanes are added pair by pair; the NR x MR sums of a
 // warp are spread over its lanes while they are added (a lane passes on half of what it holds at each step), so that 32 sums
-// take 31 exchanges and every lane stores one of them.
-constexpr int NR = 4;
-template <int MR>
+// take 31 exchanges and every lane stores one of them.  NORM: every block normalises the few short rows of A into shared memory
+// for itself, a launch less on a chain that is nothing but launches.
+constexpr int NR = 4, NORM_MAX = 4096;
+template <int MR, bool NORM>
 __global__ void __launch_bounds__(256, MR == 8 ? 1 : 2) gemm_f32_rows_kernel(GemmArgs g) {
   const int lane = threadIdx.x & 31;
   const long long n0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * NR;
-  if (n0 >= g.N) return;
   const float* A = reinterpret_cast<const float*>(g.A);
+  long long lda = g.lda;
+  if (NORM) {
+    __shared__ __align__(16) float rows[NORM ? NORM_MAX : 4];
+    for (int m = threadIdx.x >> 5; m < g.M; m += blockDim.x >> 5) {
+      float ss = 0.f;
+      for (int k = lane * 4; k < g.K; k += 128) {
+        const float4 x = *reinterpret_cast<const float4*>(A + m * lda + k);
+        ss += x.x * x.x; ss += x.y * x.y; ss += x.z * x.z; ss += x.w * x.w;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float r = sqrtf(ss / (float)g.K + g.norm_eps);
+      for (int k = lane * 4; k < g.K; k += 128) {
+        const float4 x = *reinterpret_cast<const float4*>(A + m * lda + k), w = *reinterpret_cast<const float4*>(g.norm + k);
+        *reinterpret_cast<float4*>(rows + m * g.K + k) = make_float4(x.x / r * w.x, x.y / r * w.y, x.z / r * w.z, x.w / r * w.w);
+      }
+    }
+    __syncthreads();
+    A = rows; lda = g.K;
+  }
+  if (n0 >= g.N) return;
   const float* wr[NR];
 #pragma unroll
   for (int j = 0; j < NR; ++j) wr[j] = reinterpret_cast<const float*>(g.W) + (n0 + j < g.N ? n0 + j : g.N - 1) * g.ldw;
@@ -182,7 +203,7 @@ __global__ void __launch_bounds__(256, MR == 8 ? 1 : 2) gemm_f32_rows_kernel(Gem
 #pragma unroll
       for (int i = 0; i < MR; ++i) {
         const int m = m0 + i < g.M ? m0 + i : g.M - 1;
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(A + (long long)m * g.lda + k);
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(A + m * lda + k);
 #pragma unroll
         for (int j = 0; j < NR; ++j) {
           fma2(acc[j * MR + i], x.x, wv[j].x);
@@ -232,15 +253,25 @@ template <int MR>
 inline int32_t launch_rows(vn_ctx* ctx, const GemmArgs& g) {
   // blocks of two warps while that leaves SMs without one, of eight where the matrix is large
   const int warps = g.N >= 8 * NR * 4 * ctx->sm_count ? 8 : 2;
-  VN_LAUNCH_NAMED(ctx, g.tag ? g.tag : "gemm_f32_rows_kernel", gemm_f32_rows_kernel<MR>, ceil_div(g.N, warps * NR), warps * 32, 0, g);
+  const char* name = g.tag ? g.tag : "gemm_f32_rows_kernel";
+  if (g.norm) VN_LAUNCH_NAMED(ctx, name, (gemm_f32_rows_kernel<MR, true>), ceil_div(g.N, warps * NR), warps * 32, 0, g);
+  else VN_LAUNCH_NAMED(ctx, name, (gemm_f32_rows_kernel<MR, false>), ceil_div(g.N, warps * NR), warps * 32, 0, g);
   return VN_OK;
 }
 
 }  // namespace f32_detail
 
+// GEMMs that may ask for the norm of their rows: the rows kernel's, with few short rows.  The step of 5 rows through the 64-wide
+// model took 89 us with 19 launches; a norm launch is 3 us of it, the norm itself inside a GEMM of 5 x 64 values under 1 us.
+inline bool gemm_f32_norm_supported(const GemmArgs& g) {
+  return g.M <= 16 && (long long)g.M * g.K <= f32_detail::NORM_MAX && g.K > 0 && g.nseg == 1 && !g.seg_cnt && !g.a_rows && !g.wq && g.ldw_k == 1 &&
+         (((uintptr_t)g.A | (uintptr_t)(g.lda * 4) | (uintptr_t)g.W | (uintptr_t)(g.ldw * 4) | (uintptr_t)(g.K * 4)) & 15) == 0 && ((uintptr_t)g.norm & 15) == 0;
+}
+
 inline int32_t launch_gemm_f32(vn_ctx* ctx, const GemmArgs& g) {
   using namespace f32_detail;
   if (g.M <= 0 || g.N <= 0) return VN_OK;
+  if (g.norm && !gemm_f32_norm_supported(g)) return vn_fail(ctx, VN_ERR_UNSUPPORTED, "norm inside an fp32 GEMM of %d x %d", g.M, g.K);
   const bool aligned_a = (((uintptr_t)g.A | (uintptr_t)(g.lda * 4) | (uintptr_t)(g.a_stride * 4) | (uintptr_t)(g.K * 4)) & 15) == 0;
   const bool aligned_w = g.ldw_k == 1 && (((uintptr_t)g.W | (uintptr_t)(g.ldw * 4) | (uintptr_t)(g.w_stride * 4) | (uintptr_t)(g.K * 4)) & 15) == 0;
   // A warp per four features streams the weights once where few rows meet them; up to 16 rows also for narrow matrices, where the

@@ -528,23 +528,31 @@ int32_t forward_t(vn_model* m, vn_kv* kv, const int64_t* tokens, int B, int Tn, 
       g.W = dense;
     }
   };
+  // the GEMM normalises its rows itself where it can (few short rows of an fp32 model), else the norm's own kernel runs first
+  auto normed = [&](GemmArgs& g, const float* w, long long row_mul, long long row_add, float* out32) -> int32_t {
+    if (std::is_same<T, float>::value && !out32 && !g.wq) {
+      GemmArgs f = g;
+      f.A = m->x + row_add * D; f.lda = row_mul * D; f.norm = w; f.norm_eps = 1e-6f;
+      if (gemm_f32_norm_supported(f)) { g = f; return VN_OK; }
+    }
+    VN_LAUNCH(ctx, rmsnorm_kernel<T>, g.M, 256, 0, m->x, w, (T*)m->h, out32, (int)row_mul, (int)row_add, D, 1e-6f);
+    return VN_OK;
+  };
   VN_LAUNCH(ctx, embed_kernel<T>, M, 128, 0, (const long long*)tokens, (const T*)m->emb, m->x, D, c.vocab, emb_scale,
             m->status);
   for (int li = 0; li < c.n_layer; ++li) {
     Layer& L = m->layers[li];
-    VN_LAUNCH(ctx, rmsnorm_kernel<T>, M, 256, 0, m->x, L.norm1, (T*)m->h, (float*)nullptr, 1, 0, D, 1e-6f);
     GemmArgs g;
     if (is_delta(L.kind)) {
+      VN_LAUNCH(ctx, rmsnorm_kernel<T>, M, 256, 0, m->x, L.norm1, (T*)m->h, (float*)nullptr, 1, 0, D, 1e-6f);
       TRY(delta_attention<T>(m, kv, L, B, Tn, tree, slot_offset));
     } else {
     const int pr = m->pair0[li];
     g.A = m->h; g.lda = D; g.W = L.wqkv; g.ldw = D; g.C = m->qkv; g.ldc = qkv_ld; g.M = M; g.N = qkv_ld; g.K = D;
     g.tag = "gemm_qkv";
     pick(g, L.wqkv, L.q[0], L.qs[0], 0);
+    TRY(normed(g, L.norm1, 1, 0, nullptr));
     TRY(linear(m, g));
-    VN_LAUNCH(ctx, rope_append_kernel<T>, M, 128, 0, m->qkv, m->rope_cos, m->rope_sin, kv->lens,
-              tree ? m->depth_dev : (const int*)nullptr, (T*)kv->k[pr], (T*)kv->v[pr], Tn, H, n_kv, hd, kv->max_seq,
-              c.use_rope, m->rope_rows, slot_offset);
     AttnArgs a;
     a.q = m->qkv; a.ld_q = qkv_ld; a.kc = kv->k[pr]; a.vc = kv->v[pr]; a.sink_k = L.sink_k; a.sink_v = L.sink_v;
     a.out = m->attn; a.lens = kv->lens; a.depth = tree ? m->depth_dev : nullptr; a.anc = tree ? m->anc_dev : nullptr;
@@ -555,7 +563,17 @@ int32_t forward_t(vn_model* m, vn_kv* kv, const int64_t* tokens, int B, int Tn, 
     a.g_b = 1.f / (1.f + expf(-L.gate_logits[1]));
     a.g_c = 1.f / (1.f + expf(-L.gate_logits[2]));
     a.scale = 1.0f / sqrtf((float)hd);
-    if (attn_prefill_supported(a, c.bf16 != 0) && !m->force_simt_attn) {
+    const bool prefill = attn_prefill_supported(a, c.bf16 != 0) && !m->force_simt_attn;
+    // few new rows on the rows kernel: its blocks rotate and append them (a prompt's rows are read by many blocks, each of
+    // which would rotate them again)
+    if (Tn <= 16 && !prefill && !(attn_mma_supported(a, c.bf16 != 0) && !m->force_simt_attn) && trisparse_plan(ctx, a, B).rows) {
+      a.fresh = 1; a.cos_t = m->rope_cos; a.sin_t = m->rope_sin; a.use_rope = c.use_rope; a.rope_rows = m->rope_rows;
+    } else {
+      VN_LAUNCH(ctx, rope_append_kernel<T>, M, 128, 0, m->qkv, m->rope_cos, m->rope_sin, kv->lens,
+                tree ? m->depth_dev : (const int*)nullptr, (T*)kv->k[pr], (T*)kv->v[pr], Tn, H, n_kv, hd, kv->max_seq,
+                c.use_rope, m->rope_rows, slot_offset);
+    }
+    if (prefill) {
       TRY(launch_attn_prefill(ctx, a, B));
     } else if (attn_mma_supported(a, c.bf16 != 0) && !m->force_simt_attn) {
       TRY(launch_attn_mma(ctx, a, B));
@@ -569,13 +587,13 @@ int32_t forward_t(vn_model* m, vn_kv* kv, const int64_t* tokens, int B, int Tn, 
     pick(g, L.wproj, L.q[1], L.qs[1], 0);
     TRY(linear(m, g));
     const bool mod = L.kind == 1;
-    VN_LAUNCH(ctx, rmsnorm_kernel<T>, M, 256, 0, m->x, L.norm2, (T*)m->h, mod ? m->h32 : (float*)nullptr,
-              1, 0, D, 1e-6f);
+    if (mod) VN_LAUNCH(ctx, rmsnorm_kernel<T>, M, 256, 0, m->x, L.norm2, (T*)m->h, m->h32, 1, 0, D, 1e-6f);
     if (!mod) {
       g = GemmArgs();
       g.A = m->h; g.lda = D; g.W = L.w_gateup; g.ldw = D; g.C = m->act; g.ldc = c.mlp_hidden; g.M = M;
       g.N = 2 * c.mlp_hidden; g.K = D; g.epi = EPI_SWIGLU; g.c_bf16 = c.bf16; g.tag = "gemm_gateup";
       pick(g, L.w_gateup, L.q[2], L.qs[2], 0);
+      TRY(normed(g, L.norm2, 1, 0, nullptr));
       TRY(linear(m, g));
       g = GemmArgs();
       g.A = m->act; g.lda = c.mlp_hidden; g.W = L.w_down; g.ldw = c.mlp_hidden; g.C = m->x; g.ldc = D; g.M = M; g.N = D;
@@ -647,13 +665,15 @@ int32_t forward_t(vn_model* m, vn_kv* kv, const int64_t* tokens, int B, int Tn, 
   // final norm + head on every row, or on the last position of every sequence
   const int rows_out = last_only ? B : M;
   const int row_mul = last_only ? Tn : 1, row_add = last_only ? Tn - 1 : 0;
-  VN_LAUNCH(ctx, rmsnorm_kernel<T>, rows_out, 256, 0, m->x, m->norm_f, (T*)m->h, out_hidden, row_mul, row_add, D, 1e-6f);
+  GemmArgs g;
+  g.A = m->h; g.lda = D; g.W = m->head; g.ldw = D; g.C = out_logits; g.ldc = c.vocab; g.M = rows_out; g.N = c.vocab;
+  g.K = D; g.tag = "gemm_head";
   if (out_logits) {
-    GemmArgs g;
-    g.A = m->h; g.lda = D; g.W = m->head; g.ldw = D; g.C = out_logits; g.ldc = c.vocab; g.M = rows_out; g.N = c.vocab;
-    g.K = D; g.tag = "gemm_head";
     pick(g, m->head, m->head_q, m->head_qs, 0);
+    TRY(normed(g, m->norm_f, row_mul, row_add, out_hidden));
     TRY(linear(m, g));
+  } else {
+    VN_LAUNCH(ctx, rmsnorm_kernel<T>, rows_out, 256, 0, m->x, m->norm_f, (T*)m->h, out_hidden, row_mul, row_add, D, 1e-6f);
   }
   return VN_OK;
 }

@@ -179,6 +179,9 @@ struct AttnArgs {
   const float* cos_t = nullptr;
   const float* sin_t = nullptr;
   int use_rope = 0, rope_rows = 0;
+  // Rows kernel only: k and v of the new positions still stand behind q in its rows (columns (H + kv head) hd and (H + n_kv + kv
+  // head) hd) and q is not rotated yet; the blocks rotate what they read and append their own rows' k and v to the cache.
+  int fresh = 0;
   // Tensor-core kernel only: a module of the delta attention family (verse_nex/delta_attention.py) on the same three
   // passes.  delta 1 = DSA (window + sinks + dense), 2 = KDA (one pass over all keys with the window | anchor mask),
   // 3 = GMLA (dense, or the window beyond alibi_max keys); the dense pass is the ALiBi pass without its bias and the
@@ -402,14 +405,46 @@ __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, 
   const int nk = max(0, min(hi - lo, cap - a.n_sink)), total = nk + a.n_sink;
   const long long kstride = (long long)a.n_kv * hd, base = ((long long)b * a.max_seq * a.n_kv + kvh) * hd;
 
+  // four dims of a new position's q or k (x: its row, d: the first of them), rotated
+  auto rotated = [&](const float* x, int d, int t) {
+    float4 v = *reinterpret_cast<const float4*>(x + d);
+    if (a.use_rope) {
+      const int half = hd >> 1, p = min(len + (a.depth ? a.depth[t] : t), a.rope_rows - 1), j = d < half ? d : d - half;
+      const float4 o = *reinterpret_cast<const float4*>(x + (d < half ? d + half : d - half));
+      const float4 c = *reinterpret_cast<const float4*>(a.cos_t + (long long)p * half + j), s = *reinterpret_cast<const float4*>(a.sin_t + (long long)p * half + j);
+      const float g = d < half ? -1.f : 1.f;
+      v = make_float4(v.x * c.x + g * o.x * s.x, v.y * c.y + g * o.y * s.y, v.z * c.z + g * o.z * s.z, v.w * c.w + g * o.w * s.w);
+    }
+    return v;
+  };
+  // the same of its k (which 0) or v (which 1) as the cache holds it
+  auto appended = [&](int which, int t, int d) {
+    const float* x = a.q + (long long)(b * a.Tn + t) * a.ld_q + (a.H + which * a.n_kv + kvh) * hd;
+    const float4 v = which ? *reinterpret_cast<const float4*>(x + d) : rotated(x, d, t);
+    T r[4] = {from_f<T>(v.x), from_f<T>(v.y), from_f<T>(v.z), from_f<T>(v.w)};
+    return make_float4(ld_f(r), ld_f(r + 1), ld_f(r + 2), ld_f(r + 3));
+  };
+  if (a.fresh)
+    for (int e = tid; e < 2 * (t_last - t_first + 1) * nq; e += TR_THREADS) {
+      const int which = e & 1, t = t_first + (e >> 1) / nq, d = ((e >> 1) % nq) * 4, slot = len + t;
+      if (slot >= a.max_seq) continue;
+      const float4 v = appended(which, t, d);
+      T* dst = reinterpret_cast<T*>(const_cast<void*>(which ? a.vc : a.kc)) + base + (long long)slot * kstride + d;
+      dst[0] = from_f<T>(v.x); dst[1] = from_f<T>(v.y); dst[2] = from_f<T>(v.z); dst[3] = from_f<T>(v.w);
+    }
+
   // a tile's rows: TR_TILE * nq float4s over the threads, at most 8 each (hd <= 64)
   float4 pre[8];
-  auto fetch = [&](const void* cache, const void* sink, int j0) {
+  auto fetch = [&](int which, int j0) {
+    const void* cache = which ? a.vc : a.kc;
+    const void* sink = which ? a.sink_v : a.sink_k;
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int e = tid + u * TR_THREADS, r = e / nq, d = (e % nq) * 4, j = j0 + r;
       pre[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < TR_TILE && j < total) {
+      if (r < TR_TILE && j < nk && a.fresh && lo + j >= len) {
+        pre[u] = appended(which, lo + j - len, d);
+      } else if (r < TR_TILE && j < total) {
         const T* src = j < nk ? reinterpret_cast<const T*>(cache) + base + (long long)(lo + j) * kstride
                               : reinterpret_cast<const T*>(sink) + (long long)(j - nk) * kstride + (long long)kvh * hd;
         pre[u] = load4(src + d);
@@ -423,19 +458,22 @@ __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, 
       if (r < TR_TILE) *reinterpret_cast<float4*>(sT + r * ld + d) = pre[u];
     }
   };
-  fetch(a.kc, a.sink_k, 0);
+  fetch(0, 0);
   for (int e = tid; e < R * nq; e += TR_THREADS) {
     const int i = i0 + e / nq, d = (e % nq) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i < n_items) v = *reinterpret_cast<const float4*>(a.q + (long long)(b * a.Tn + i / n_rep) * a.ld_q + (kvh * n_rep + i % n_rep) * hd + d);
+    if (i < n_items) {
+      const float* x = a.q + (long long)(b * a.Tn + i / n_rep) * a.ld_q + (kvh * n_rep + i % n_rep) * hd;
+      v = a.fresh ? rotated(x, d, i / n_rep) : *reinterpret_cast<const float4*>(x + d);
+    }
     *reinterpret_cast<float4*>(sQ + e * 4) = v;
   }
   // ---- scores: a thread has one key of the tile and half of the rows
   for (int j0 = 0; j0 < total; j0 += TR_TILE) {
     put();
     __syncthreads();
-    if (j0 + TR_TILE < total) fetch(a.kc, a.sink_k, j0 + TR_TILE);
-    else fetch(a.vc, a.sink_v, 0);
+    if (j0 + TR_TILE < total) fetch(0, j0 + TR_TILE);
+    else fetch(1, 0);
     const int r = tid & (TR_TILE - 1), h0 = (tid / TR_TILE) * (R / 2);
     float s[R / 2];
 #pragma unroll
@@ -514,7 +552,7 @@ __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, 
   for (int j0 = 0; j0 < total; j0 += TR_TILE) {
     put();
     __syncthreads();
-    if (j0 + TR_TILE < total) fetch(a.vc, a.sink_v, j0 + TR_TILE);
+    if (j0 + TR_TILE < total) fetch(1, j0 + TR_TILE);
     if (slice < slices) {
       const int n = min(TR_TILE, total - j0);
 #pragma unroll 4
@@ -537,9 +575,8 @@ __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, 
   }
 }
 
-// The rows kernel where a block's scores fit shared memory, else the one-warp-per-row kernel (windows of many thousand keys).
-template <typename T>
-inline int32_t launch_trisparse(vn_ctx* ctx, const AttnArgs& a, int B) {
+struct TrisparsePlan { int R; long long cap, smem; bool rows; };
+inline TrisparsePlan trisparse_plan(const vn_ctx* ctx, const AttnArgs& a, int B) {
   const int n_rep = a.H / a.n_kv, n_items = a.Tn * n_rep;
   // eight rows a block once that gives two blocks per SM, four (shorter soft-maxes per warp) before
   const int R = (long long)ceil_div(n_items, 8) * a.n_kv * B >= 2ll * ctx->sm_count ? 8 : 4;
@@ -549,7 +586,16 @@ inline int32_t launch_trisparse(vn_ctx* ctx, const AttnArgs& a, int B) {
   if (a.use_alibi && a.alibi_window == 0) keys = std::max(keys, std::min<long long>(a.max_seq, (long long)a.alibi_max + grown));
   const long long cap = (keys + a.n_sink) | 1;
   const long long smem = (TR_TILE * (a.hd + 4) + R * a.hd + R * cap) * 4;
-  if (smem > 160 * 1024 || B > 65535 || a.n_kv > 65535) {
+  return {R, cap, smem, smem <= 160 * 1024 && B <= 65535 && a.n_kv <= 65535};
+}
+
+// The rows kernel where a block's scores fit shared memory, else the one-warp-per-row kernel (windows of many thousand keys).
+template <typename T>
+inline int32_t launch_trisparse(vn_ctx* ctx, const AttnArgs& a, int B) {
+  const TrisparsePlan p = trisparse_plan(ctx, a, B);
+  const int R = p.R, n_items = a.Tn * (a.H / a.n_kv);
+  const long long cap = p.cap, smem = p.smem;
+  if (!p.rows) {
     dim3 grid(ceil_div(a.H, 8), B * a.Tn);
     VN_LAUNCH(ctx, trisparse_attn_kernel<T>, grid, 256, 0, a);
     return VN_OK;
