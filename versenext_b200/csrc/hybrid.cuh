@@ -1353,7 +1353,7 @@ int32_t mixture(vn_model* m, const HLayer& L, int M, const Buffers& b, const Nex
   if (tc) {
     int *off = b.sub_seg, *cnt = off + b.sub_cap, *w = cnt + b.sub_cap;
     VN_LAUNCH(ctx, mod_subseg_kernel, 1, 32, 0, (const int*)hm.exp_count, (const int*)hm.exp_off, mats, off, cnt, w, b.sub_cap, 256);
-    VN_LAUNCH(ctx, gather_sorted_kernel<T>, M * S, 128, 0, (const T*)m->h, (const int*)b.sorted_row, (T*)b.hs, D, sorted_w);
+    VN_LAUNCH(ctx, gather_sorted_kernel<T>, ceil_div(M * S, 4), 128, 0, (const T*)m->h, (const int*)b.sorted_row, (T*)b.hs, D, sorted_w, M * S);
     TRY(ensure_partial(m, 1024));
     for (GemmArgs* g : {&up, &down}) {
       g->M = 256; g->seg_off = off; g->seg_cnt = cnt; g->seg_w = w; g->n_w = mats; g->nseg = b.sub_cap;
@@ -1363,7 +1363,7 @@ int32_t mixture(vn_model* m, const HLayer& L, int M, const Buffers& b, const Nex
     }
   } else {                                                // the kernels of any shape gather rows themselves, as they are
     if (scale) {
-      VN_LAUNCH(ctx, gather_sorted_kernel<T>, M * S, 128, 0, (const T*)m->h, (const int*)b.sorted_row, (T*)b.hs, D, sorted_w);
+      VN_LAUNCH(ctx, gather_sorted_kernel<T>, ceil_div(M * S, 4), 128, 0, (const T*)m->h, (const int*)b.sorted_row, (T*)b.hs, D, sorted_w, M * S);
     } else {
       up.A = m->h; up.a_rows = b.sorted_row;
     }

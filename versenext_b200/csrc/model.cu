@@ -623,7 +623,7 @@ int32_t forward_t(vn_model* m, vn_kv* kv, const int64_t* tokens, int B, int Tn, 
         int* sub_off = m->sub_seg; int* sub_cnt = m->sub_seg + m->sub_cap; int* sub_w = m->sub_seg + 2 * m->sub_cap;
         VN_LAUNCH(ctx, mod_subseg_kernel, 1, 32, 0, (const int*)m->expert_count, (const int*)m->expert_off, ne, sub_off,
                   sub_cnt, sub_w, n_sub, piece);
-        VN_LAUNCH(ctx, gather_sorted_kernel<T>, M * S, 128, 0, (const T*)m->h, (const int*)m->sorted_row, (T*)m->hs, D, (const float*)nullptr);
+        VN_LAUNCH(ctx, gather_sorted_kernel<T>, ceil_div(M * S, 4), 128, 0, (const T*)m->h, (const int*)m->sorted_row, (T*)m->hs, D, (const float*)nullptr, M * S);
         TRY(ensure_partial(m, 1024));
         TcPlan plan;
         plan.error_flag = m->tc_error;

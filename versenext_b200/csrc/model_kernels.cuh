@@ -88,8 +88,23 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
   __shared__ float sm[8];
   const long long src = (long long)blockIdx.x * row_mul + row_add;   // e.g. the last position of every sequence
   const float* xr = x + src * D;
+  // rows of up to 4096 values on 16-byte boundaries stay in registers: one read, four values a load (4096 rows of 1024 took 9 us
+  // with a scalar read for the sum and another for the result)
+  const bool vec = D <= 4096 && (D & 3) == 0 && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)y32) & 15) == 0;
+  float4 v[4];
   float ss = 0.f;
-  for (int d = threadIdx.x; d < D; d += 256) ss += xr[d] * xr[d];
+  if (vec) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int d = (threadIdx.x + u * 256) * 4;
+      if (d < D) v[u] = load4(xr + d);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if ((threadIdx.x + u * 256) * 4 < D) ss += v[u].x * v[u].x + v[u].y * v[u].y + v[u].z * v[u].z + v[u].w * v[u].w;
+  } else {
+    for (int d = threadIdx.x; d < D; d += 256) ss += xr[d] * xr[d];
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = ss;
@@ -98,6 +113,17 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
 #pragma unroll
   for (int i = 0; i < 8; ++i) tot += sm[i];
   const float r = sqrtf(tot / (float)D + eps);
+  if (vec) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int d = (threadIdx.x + u * 256) * 4;
+      if (d >= D) break;
+      const float4 f = load4(w + d), o = make_float4(v[u].x / r * f.x, v[u].y / r * f.y, v[u].z / r * f.z, v[u].w / r * f.w);
+      if (y) store4(y + (long long)blockIdx.x * D + d, o);
+      if (y32) store4(y32 + (long long)blockIdx.x * D + d, o);
+    }
+    return;
+  }
   for (int d = threadIdx.x; d < D; d += 256) {
     const float v = xr[d] / r * w[d];
     if (y) y[(long long)blockIdx.x * D + d] = from_f<T>(v);
@@ -121,31 +147,33 @@ __global__ void rope_append_kernel(float* __restrict__ qkv, const float* __restr
   const int ld = (H + 2 * n_kv) * hd;
   float* r = qkv + (long long)row * ld;
   const int p = pos < rope_rows ? pos : rope_rows - 1;
-  // q and k heads: pairs (j, j + half)
-  const int n_rot = (H + n_kv) * half;
-  for (int i = threadIdx.x; i < n_rot; i += blockDim.x) {
-    const int head = i / half, j = i % half;
-    float x1 = r[head * hd + j], x2 = r[head * hd + half + j];
-    float o1 = x1, o2 = x2;
+  // q and k heads: four pairs (j, j + half) per thread (hd is a multiple of 8), v four values: memory-bound, 4096 rows of 24 rotated
+  // and 8 plain heads of 64 took 14 us value by value
+  const int h4 = half >> 2;
+  for (int i = threadIdx.x; i < (H + n_kv) * h4; i += blockDim.x) {
+    const int head = i / h4, j = (i % h4) * 4;
+    const float4 x1 = *reinterpret_cast<const float4*>(r + head * hd + j), x2 = *reinterpret_cast<const float4*>(r + head * hd + half + j);
+    float4 o1 = x1, o2 = x2;
     if (use_rope) {
-      const float c = cos_t[(long long)p * half + j], s = sin_t[(long long)p * half + j];
-      o1 = x1 * c + (-x2) * s;
-      o2 = x2 * c + x1 * s;
+      const float4 c = *reinterpret_cast<const float4*>(cos_t + (long long)p * half + j), s = *reinterpret_cast<const float4*>(sin_t + (long long)p * half + j);
+      o1 = make_float4(x1.x * c.x + (-x2.x) * s.x, x1.y * c.y + (-x2.y) * s.y, x1.z * c.z + (-x2.z) * s.z, x1.w * c.w + (-x2.w) * s.w);
+      o2 = make_float4(x2.x * c.x + x1.x * s.x, x2.y * c.y + x1.y * s.y, x2.z * c.z + x1.z * s.z, x2.w * c.w + x1.w * s.w);
     }
     if (head < H) {
-      r[head * hd + j] = o1;
-      r[head * hd + half + j] = o2;
+      if (use_rope) {
+        *reinterpret_cast<float4*>(r + head * hd + j) = o1;
+        *reinterpret_cast<float4*>(r + head * hd + half + j) = o2;
+      }
     } else if (slot < max_seq) {
-      const int kh = head - H;
-      T* dst = kc + (((long long)b * max_seq + slot) * n_kv + kh) * hd;
-      dst[j] = from_f<T>(o1);
-      dst[half + j] = from_f<T>(o2);
+      T* dst = kc + (((long long)b * max_seq + slot) * n_kv + head - H) * hd;
+      store4(dst + j, o1);
+      store4(dst + half + j, o2);
     }
   }
   if (slot < max_seq) {
     const float* v = r + (H + n_kv) * hd;
     T* dst = vc + ((long long)b * max_seq + slot) * n_kv * hd;
-    for (int i = threadIdx.x; i < n_kv * hd; i += blockDim.x) dst[i] = from_f<T>(v[i]);
+    for (int i = threadIdx.x * 4; i < n_kv * hd; i += blockDim.x * 4) store4(dst + i, *reinterpret_cast<const float4*>(v + i));
   }
 }
 
@@ -386,7 +414,8 @@ __global__ void __launch_bounds__(256) trisparse_attn_kernel(AttnArgs a) {
 // models have few rows and a warp that walks the keys alone (the kernel above) spends its time in a chain of exponentials,
 // 8 to 20 us a layer where this one takes 4 to 9 (float32, 64 wide heads, 5 rows at context 32, 2 x 300 rows of prompts).
 constexpr int TR_TILE = 64, TR_THREADS = 128;
-template <typename T, int R>
+// FRESH: AttnArgs::fresh, apart because the code for it costs the prompts 2 % (282 -> 288 us for 2 x 300 rows)
+template <typename T, int R, bool FRESH>
 __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, int cap) {
   extern __shared__ __align__(16) float tr_smem[];
   const int hd = a.hd, nq = hd >> 2, ld = hd + 4;
@@ -424,7 +453,7 @@ __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, 
     T r[4] = {from_f<T>(v.x), from_f<T>(v.y), from_f<T>(v.z), from_f<T>(v.w)};
     return make_float4(ld_f(r), ld_f(r + 1), ld_f(r + 2), ld_f(r + 3));
   };
-  if (a.fresh)
+  if (FRESH)
     for (int e = tid; e < 2 * (t_last - t_first + 1) * nq; e += TR_THREADS) {
       const int which = e & 1, t = t_first + (e >> 1) / nq, d = ((e >> 1) % nq) * 4, slot = len + t;
       if (slot >= a.max_seq) continue;
@@ -442,7 +471,7 @@ __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, 
     for (int u = 0; u < 8; ++u) {
       const int e = tid + u * TR_THREADS, r = e / nq, d = (e % nq) * 4, j = j0 + r;
       pre[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < TR_TILE && j < nk && a.fresh && lo + j >= len) {
+      if (r < TR_TILE && FRESH && j < nk && lo + j >= len) {
         pre[u] = appended(which, lo + j - len, d);
       } else if (r < TR_TILE && j < total) {
         const T* src = j < nk ? reinterpret_cast<const T*>(cache) + base + (long long)(lo + j) * kstride
@@ -464,7 +493,7 @@ __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, 
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < n_items) {
       const float* x = a.q + (long long)(b * a.Tn + i / n_rep) * a.ld_q + (kvh * n_rep + i % n_rep) * hd;
-      v = a.fresh ? rotated(x, d, i / n_rep) : *reinterpret_cast<const float4*>(x + d);
+      v = FRESH ? rotated(x, d, i / n_rep) : *reinterpret_cast<const float4*>(x + d);
     }
     *reinterpret_cast<float4*>(sQ + e * 4) = v;
   }
@@ -601,14 +630,13 @@ inline int32_t launch_trisparse(vn_ctx* ctx, const AttnArgs& a, int B) {
     return VN_OK;
   }
   dim3 grid(ceil_div(n_items, R), a.n_kv, B);
-  if (R == 8) {
-    if (smem > 48 * 1024) VN_CUDA(ctx, cudaFuncSetAttribute(trisparse_rows_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    VN_LAUNCH(ctx, (trisparse_rows_kernel<T, 8>), grid, TR_THREADS, smem, a, (int)cap);
-  } else {
-    if (smem > 48 * 1024) VN_CUDA(ctx, cudaFuncSetAttribute(trisparse_rows_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    VN_LAUNCH(ctx, (trisparse_rows_kernel<T, 4>), grid, TR_THREADS, smem, a, (int)cap);
-  }
-  return VN_OK;
+  auto launch = [&](auto kernel) -> int32_t {
+    if (smem > 48 * 1024) VN_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    VN_LAUNCH_NAMED(ctx, "trisparse_rows_kernel", kernel, grid, TR_THREADS, smem, a, (int)cap);
+    return VN_OK;
+  };
+  if (a.fresh) return R == 8 ? launch(trisparse_rows_kernel<T, 8, true>) : launch(trisparse_rows_kernel<T, 4, true>);
+  return R == 8 ? launch(trisparse_rows_kernel<T, 8, false>) : launch(trisparse_rows_kernel<T, 4, false>);
 }
 
 // ---- MoD routing (mod.py:340-387, :748-770) ----------------------------------------------------------
@@ -740,22 +768,51 @@ __global__ void mod_scatter_kernel(const int* __restrict__ slot_expert, const in
 }
 
 // x[row] += sum_p part_w[p] * (sum_j slot_w[p, j] * y[slot_pos[p, j]])   (mod.py:196-211, :604-605, :779-781)
-__global__ void mod_combine_kernel(float* __restrict__ x, const float* __restrict__ y, const int* __restrict__ slot_pos,
-                                   const float* __restrict__ slot_w, const float* __restrict__ part_w, int D, int P,
-                                   int top_k) {
-  const int row = blockIdx.x;
-  const int S = P * top_k;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float out = 0.f;
-    for (int p = 0; p < P; ++p) {
-      float comb = 0.f;
-      for (int j = 0; j < top_k; ++j) {
-        const long long s = (long long)row * S + p * top_k + j;
-        comb += y[(long long)slot_pos[s] * D + d] * slot_w[s];
+// HBM-bound (P * top_k rows of fp32 per token).  A thread has four dims and fetches up to eight slots' rows before it adds the
+// first: 4096 tokens of 8 slots and 1024 dims 63 us with a load per value, one slot after another.
+__global__ void __launch_bounds__(256) mod_combine_kernel(float* __restrict__ x, const float* __restrict__ y, const int* __restrict__ slot_pos,
+                                                          const float* __restrict__ slot_w, const float* __restrict__ part_w, int D, int P,
+                                                          int top_k) {
+  constexpr int AHEAD = 8;
+  const int row = blockIdx.x, S = P * top_k;
+  const int* pos = slot_pos + (long long)row * S;
+  const float* w = slot_w + (long long)row * S;
+  const float* pw = part_w + (long long)row * P;
+  float* xr = x + (long long)row * D;
+  for (int d = threadIdx.x * 4; d < D; d += blockDim.x * 4) {
+    if (D % 4) {                                             // rows start anywhere: value by value
+      for (int e = d; e < min(d + 4, D); ++e) {
+        float out = 0.f;
+        for (int p = 0; p < P; ++p) {
+          float comb = 0.f;
+          for (int j = 0; j < top_k; ++j) comb += y[(long long)pos[p * top_k + j] * D + e] * w[p * top_k + j];
+          out += comb * pw[p];
+        }
+        xr[e] += out;
       }
-      out += comb * part_w[(long long)row * P + p];
+      continue;
     }
-    x[(long long)row * D + d] += out;
+    float4 out = make_float4(0.f, 0.f, 0.f, 0.f), comb = out, v[AHEAD];
+    float4 old = *reinterpret_cast<const float4*>(xr + d);
+    int p = 0, j = 0;
+    for (int s0 = 0; s0 < S; s0 += AHEAD) {
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u)
+        if (s0 + u < S) v[u] = *reinterpret_cast<const float4*>(y + (long long)pos[s0 + u] * D + d);
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        if (s0 + u >= S) break;
+        const float f = w[s0 + u];
+        comb.x += v[u].x * f; comb.y += v[u].y * f; comb.z += v[u].z * f; comb.w += v[u].w * f;
+        if (++j == top_k) {
+          const float g = pw[p++];
+          out.x += comb.x * g; out.y += comb.y * g; out.z += comb.z * g; out.w += comb.w * g;
+          comb = make_float4(0.f, 0.f, 0.f, 0.f);
+          j = 0;
+        }
+      }
+    }
+    *reinterpret_cast<float4*>(xr + d) = make_float4(old.x + out.x, old.y + out.y, old.z + out.z, old.w + out.w);
   }
 }
 
@@ -996,22 +1053,34 @@ __global__ void mod_dispatch_kernel(const T* __restrict__ src, const int* __rest
 // sorted_w: a factor per copied row, or null.  Rows that are not whole 16-byte pieces go element by element.
 template <typename T>
 __global__ void gather_sorted_kernel(const T* __restrict__ src, const int* __restrict__ sorted_row, T* __restrict__ dst,
-                                     int D, const float* __restrict__ sorted_w) {
+                                     int D, const float* __restrict__ sorted_w, int n_rows) {
   pdl_trigger();
   pdl_wait();
-  const long long s = sorted_row[blockIdx.x];
-  const float f = sorted_w ? sorted_w[blockIdx.x] : 1.f;
+  // a warp per row, four 16-byte loads of a lane in flight (a block per row: 34 us for 32,768 rows of 2 KB)
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= n_rows) return;
+  const long long s = sorted_row[row];
+  const float f = sorted_w ? sorted_w[row] : 1.f;
   if (D * sizeof(T) % 16) {
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
+    for (int i = lane; i < D; i += 32) {
       const T v = src[s * D + i];
-      dst[(long long)blockIdx.x * D + i] = sorted_w ? from_f<T>(to_f<T>(v) * f) : v;
+      dst[(long long)row * D + i] = sorted_w ? from_f<T>(to_f<T>(v) * f) : v;
     }
     return;
   }
   const uint4* a = reinterpret_cast<const uint4*>(src + s * D);
-  uint4* b = reinterpret_cast<uint4*>(dst + (long long)blockIdx.x * D);
+  uint4* b = reinterpret_cast<uint4*>(dst + (long long)row * D);
   const int n16 = D * (int)sizeof(T) / 16;
-  for (int i = threadIdx.x; i < n16; i += blockDim.x) b[i] = sorted_w ? scaled16<T>(a[i], f) : a[i];
+#pragma unroll 1
+  for (int i0 = lane; i0 < n16; i0 += 128) {
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + 32 * u < n16) v[u] = a[i0 + 32 * u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + 32 * u < n16) b[i0 + 32 * u] = sorted_w ? scaled16<T>(v[u], f) : v[u];
+  }
 }
 
 // combine with split-K partials of the expert outputs: y = sum_s ypart[s]; x[row] += the weighted sum; then, if
