@@ -64,14 +64,32 @@ __device__ __forceinline__ float gelu_tanh(float x) {
   return 0.5f * x * (1.0f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x)));
 }
 // a gated feed-forward's function of gate g and up u (GluAct).  GLU_CLAMP: g capped from above, u from both sides, g sigmoid(1.702 g) (u + 1);
-// `fast`: the result is kept in 16 bits
-__device__ __forceinline__ float glu(float g, float u, int act, float limit, bool fast) {
-  if (act == GLU_CLAMP) {
+// `fast`: the result is kept in 16 bits.  There silu and gelu are x / (1 + e^-z) too: the forms with tanh lose the digits that
+// 1 + tanh cancels for negative x, and cost more.
+template <int ACT>
+__device__ __forceinline__ float glu_of(float g, float u, float limit, bool fast) {
+  if (ACT == GLU_CLAMP) {
     g = fminf(g, limit);
     const float b = fminf(fmaxf(u, -limit), limit) + 1.f;
     return (fast ? __fdividef(g, 1.0f + __expf(-1.702f * g)) : g / (1.0f + expf(-1.702f * g))) * b;
   }
-  return (act == GLU_GELU ? gelu_tanh(g) : silu_ref(g)) * u;
+  if (fast) {
+    const float z = ACT == GLU_GELU ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : g;
+    return __fdividef(g, 1.0f + __expf(-z)) * u;
+  }
+  return (ACT == GLU_GELU ? gelu_tanh(g) : silu_ref(g)) * u;
+}
+__device__ __forceinline__ float glu(float g, float u, int act, float limit, bool fast) {
+  return act == GLU_CLAMP ? glu_of<GLU_CLAMP>(g, u, limit, fast) : act == GLU_GELU ? glu_of<GLU_GELU>(g, u, limit, fast) : glu_of<GLU_SILU>(g, u, limit, fast);
+}
+template <int ACT> struct GluTag { static constexpr int act = ACT; };
+// f(GluTag) for an act known at run time: the choice stands outside f's loops, whose values then overlap (a branch per value made a
+// 32-row chunk of an epilogue 3900 cycles long)
+template <typename F>
+__device__ __forceinline__ void with_glu(int act, F f) {
+  if (act == GLU_CLAMP) f(GluTag<GLU_CLAMP>());
+  else if (act == GLU_GELU) f(GluTag<GLU_GELU>());
+  else f(GluTag<GLU_SILU>());
 }
 
 __device__ __forceinline__ float mul_at(const GemmArgs& g, long long idx) {

@@ -166,6 +166,13 @@ __device__ __forceinline__ void umma_bf16(unsigned tmem_d, unsigned long long da
 __device__ __forceinline__ void umma_commit(unsigned long long* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  unsigned p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void tmem_ld32(unsigned taddr, unsigned (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -347,20 +354,23 @@ __device__ __forceinline__ void tc_epilogue_chunk(const TcArgs& g, const unsigne
         asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
         const int c4 = lane * 4;
         if (n0 + c4 + 3 < g.N) {
-#pragma unroll 2
-          for (int j = 0; j < 8; ++j) {
-            const int row = q * 8 + j;
-            if (row < mrem) {
-              const float4 v = *reinterpret_cast<const float4*>(tile + row * BF + c4);
-              const float o0 = glu(v.x, v.y, g.act, g.act_limit, g.c_bf16), o1 = glu(v.z, v.w, g.act, g.act_limit, g.c_bf16);
-              const long long at = (long long)(row0 + m0 + row) * g.ldc + ((n0 + c4) >> 1);
-              if (g.c_bf16)
-                *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(g.C) + at) =
-                    __floats2bfloat162_rn(o0, o1);
-              else
-                *reinterpret_cast<float2*>(reinterpret_cast<float*>(g.C) + at) = make_float2(o0, o1);
+          with_glu(g.act, [&](auto tag) {
+            constexpr int ACT = decltype(tag)::act;
+#pragma unroll 4
+            for (int j = 0; j < 8; ++j) {
+              const int row = q * 8 + j;
+              if (row < mrem) {
+                const float4 v = *reinterpret_cast<const float4*>(tile + row * BF + c4);
+                const long long at = (long long)(row0 + m0 + row) * g.ldc + ((n0 + c4) >> 1);
+                if (g.c_bf16)
+                  *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(g.C) + at) =
+                      __floats2bfloat162_rn(glu_of<ACT>(v.x, v.y, g.act_limit, true), glu_of<ACT>(v.z, v.w, g.act_limit, true));
+                else
+                  *reinterpret_cast<float2*>(reinterpret_cast<float*>(g.C) + at) =
+                      make_float2(glu_of<ACT>(v.x, v.y, g.act_limit, false), glu_of<ACT>(v.z, v.w, g.act_limit, false));
+              }
             }
-          }
+          });
         }
       } else {
 #pragma unroll
@@ -377,15 +387,15 @@ __device__ __forceinline__ void tc_epilogue_chunk(const TcArgs& g, const unsigne
       const float bias = g.bias && n < g.N ? g.bias[n] : 0.f;
       if (vec_ok) {
         float* tile = reinterpret_cast<float*>(base) + buf * (32 * BF);
+        const int c4 = lane * 4;
+        float4 x[8];                                     // on their way while the tile is staged
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (n0 + c4 < g.N && q * 8 + j < mrem) x[j] = *reinterpret_cast<const float4*>(dst + (long long)(q * 8 + j) * g.ldc + c4);
 #pragma unroll
         for (int i = 0; i < 32; ++i) tile[i * BF + f] = __uint_as_float(r[i]) + bias;
         asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
-        const int c4 = lane * 4;
         if (n0 + c4 < g.N) {
-          float4 x[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (q * 8 + j < mrem) x[j] = *reinterpret_cast<const float4*>(dst + (long long)(q * 8 + j) * g.ldc + c4);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int row = q * 8 + j;

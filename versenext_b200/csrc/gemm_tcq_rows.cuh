@@ -19,13 +19,6 @@ namespace tc_detail {
 
 constexpr int QR_ROWS = 128, QR_CONV = 6, QR_WRITE = QR_CONV + 4, QR_THREADS = (2 + QR_WRITE) * 32;
 
-// one lane of a converged warp
-__device__ __forceinline__ bool elect_one() {
-  unsigned p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
-
 // eight biased nibbles (value + 8, element e in bits 4e..4e+3) -> four bf16x2 words.  0x4300 | n is the bf16 128 + n.
 __device__ __forceinline__ void i4x8_to_bf16_ints(unsigned x, unsigned (&o)[4]) {
   const __nv_bfloat162 off = __floats2bfloat162_rn(136.f, 136.f);
@@ -44,36 +37,42 @@ __device__ __forceinline__ void qr_write(const TcArgs& g, const float* tile, int
   const int c4 = lane * 4, n = n0 + c4;
   if (vec) {
     if (n >= g.N) return;                                                    // N % 4 == 0
+    auto rows = [&](auto tag) {
+      constexpr int ACT = decltype(tag)::act;
+      (void)ACT;
 #pragma unroll 1
-    for (int r0 = w; r0 < cnt; r0 += 4 * QR_WRITE) {                         // four rows at a time: loads first, then stores
-      float4 x[4];
-      if (MODE == TC_ADD) {
+      for (int r0 = w; r0 < cnt; r0 += 4 * QR_WRITE) {                         // four rows at a time: loads first, then stores
+        float4 x[4];
+        if (MODE == TC_ADD) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (r0 + QR_WRITE * j < cnt) x[j] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(g.C) + (long long)(row0 + r0 + QR_WRITE * j) * g.ldc + n);
-      }
+          for (int j = 0; j < 4; ++j)
+            if (r0 + QR_WRITE * j < cnt) x[j] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(g.C) + (long long)(row0 + r0 + QR_WRITE * j) * g.ldc + n);
+        }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = r0 + QR_WRITE * j;
-        if (r >= cnt) continue;
-        const float4 v = *reinterpret_cast<const float4*>(tile + r * BF + c4);
-        const long long at = (long long)(row0 + r) * g.ldc;
-        if (MODE == TC_SWIGLU) {
-          const float a = glu(v.x, v.y, g.act, g.act_limit, g.c_bf16), b = glu(v.z, v.w, g.act, g.act_limit, g.c_bf16);
-          if (g.c_bf16) *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(g.C) + at + (n >> 1)) = __floats2bfloat162_rn(a, b);
-          else *reinterpret_cast<float2*>(reinterpret_cast<float*>(g.C) + at + (n >> 1)) = make_float2(a, b);
-        } else if (MODE == TC_ADD) {
-          *reinterpret_cast<float4*>(reinterpret_cast<float*>(g.C) + at + n) = make_float4(x[j].x + v.x, x[j].y + v.y, x[j].z + v.z, x[j].w + v.w);
-        } else if (g.c_bf16) {
-          uint2 u;
-          *reinterpret_cast<__nv_bfloat162*>(&u.x) = __floats2bfloat162_rn(v.x, v.y);
-          *reinterpret_cast<__nv_bfloat162*>(&u.y) = __floats2bfloat162_rn(v.z, v.w);
-          *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(g.C) + at + n) = u;
-        } else {
-          *reinterpret_cast<float4*>(reinterpret_cast<float*>(g.C) + at + n) = v;
+        for (int j = 0; j < 4; ++j) {
+          const int r = r0 + QR_WRITE * j;
+          if (r >= cnt) continue;
+          const float4 v = *reinterpret_cast<const float4*>(tile + r * BF + c4);
+          const long long at = (long long)(row0 + r) * g.ldc;
+          if (MODE == TC_SWIGLU) {
+            const float a = glu_of<ACT>(v.x, v.y, g.act_limit, g.c_bf16), b = glu_of<ACT>(v.z, v.w, g.act_limit, g.c_bf16);
+            if (g.c_bf16) *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(g.C) + at + (n >> 1)) = __floats2bfloat162_rn(a, b);
+            else *reinterpret_cast<float2*>(reinterpret_cast<float*>(g.C) + at + (n >> 1)) = make_float2(a, b);
+          } else if (MODE == TC_ADD) {
+            *reinterpret_cast<float4*>(reinterpret_cast<float*>(g.C) + at + n) = make_float4(x[j].x + v.x, x[j].y + v.y, x[j].z + v.z, x[j].w + v.w);
+          } else if (g.c_bf16) {
+            uint2 u;
+            *reinterpret_cast<__nv_bfloat162*>(&u.x) = __floats2bfloat162_rn(v.x, v.y);
+            *reinterpret_cast<__nv_bfloat162*>(&u.y) = __floats2bfloat162_rn(v.z, v.w);
+            *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(g.C) + at + n) = u;
+          } else {
+            *reinterpret_cast<float4*>(reinterpret_cast<float*>(g.C) + at + n) = v;
+          }
         }
       }
-    }
+    };
+    if (MODE == TC_SWIGLU) with_glu(g.act, rows);
+    else rows(GluTag<GLU_SILU>());
     return;
   }
 #pragma unroll 1

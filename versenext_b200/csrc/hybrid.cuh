@@ -1359,7 +1359,7 @@ int32_t mixture(vn_model* m, const HLayer& L, int M, const Buffers& b, const Nex
       g->M = 256; g->seg_off = off; g->seg_cnt = cnt; g->seg_w = w; g->n_w = mats; g->nseg = b.sub_cap;
       TcPlan plan;
       plan.error_flag = m->tc_error;
-      TRY(launch_gemm_tc(ctx, *g, (long long)M * S, plan));
+      TRY(launch_gemm_many(ctx, *g, (long long)M * S, plan));
     }
   } else {                                                // the kernels of any shape gather rows themselves, as they are
     if (scale) {

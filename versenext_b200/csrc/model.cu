@@ -10,6 +10,7 @@
 #include "delta_attn.cuh"
 #include "draft_kernel.cuh"
 #include "gemm_tc.cuh"
+#include "gemm_tc2.cuh"
 #include "gemm_mma_q.cuh"
 #include "gemm_tcq.cuh"
 #include "gemm_tcq_rows.cuh"
@@ -409,7 +410,7 @@ int32_t linear(vn_model* m, GemmArgs g) {
       if (g2.nseg <= 65535 && gemm_tc_supported(g2)) {
         TcPlan plan;
         plan.error_flag = m->tc_error;
-        return launch_gemm_tc(ctx, g2, g.M, plan);
+        return launch_gemm_many(ctx, g2, g.M, plan);
       }
     }
     if (gemm_mma_supported(g)) return launch_gemm_mma(ctx, g);
@@ -633,7 +634,7 @@ int32_t forward_t(vn_model* m, vn_kv* kv, const int64_t* tokens, int B, int Tn, 
         g.seg_off = sub_off; g.seg_cnt = sub_cnt; g.seg_w = sub_w; g.n_w = ne; g.nseg = n_sub; g.tag = "gemm_expert_gateup";
         pick(g, L.e_gateup, L.q[4], L.qs[4], 2 * eh);
         if (g.wq) TRY(launch_gemm_tcq_rows(ctx, g, (long long)M * S, m->tc_error));
-        else TRY(launch_gemm_tc(ctx, g, (long long)M * S, plan));
+        else TRY(launch_gemm_many(ctx, g, (long long)M * S, plan));
         g = GemmArgs();
         g.A = m->act; g.lda = eh; g.W = L.e_down; g.ldw = eh; g.w_stride = (long long)D * eh; g.C = m->y; g.ldc = D;
         g.M = piece; g.N = D; g.K = eh; g.seg_off = sub_off; g.seg_cnt = sub_cnt; g.seg_w = sub_w; g.n_w = ne; g.nseg = n_sub;
@@ -642,7 +643,7 @@ int32_t forward_t(vn_model* m, vn_kv* kv, const int64_t* tokens, int B, int Tn, 
         TcPlan plan2;
         plan2.error_flag = m->tc_error;
         if (g.wq) TRY(launch_gemm_tcq_rows(ctx, g, (long long)M * S, m->tc_error));
-        else TRY(launch_gemm_tc(ctx, g, (long long)M * S, plan2));
+        else TRY(launch_gemm_many(ctx, g, (long long)M * S, plan2));
       } else {
       g = GemmArgs();
       g.A = m->h; g.lda = D; g.a_rows = m->sorted_row; g.W = L.e_gateup; g.ldw = D; g.w_stride = (long long)2 * eh * D;
