@@ -64,18 +64,14 @@ __device__ __forceinline__ float gelu_tanh(float x) {
   return 0.5f * x * (1.0f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x)));
 }
 // a gated feed-forward's function of gate g and up u (GluAct).  GLU_CLAMP: g capped from above, u from both sides, g sigmoid(1.702 g) (u + 1);
-// `fast`: the result is kept in 16 bits.  There silu and gelu are x / (1 + e^-z) too: the forms with tanh lose the digits that
-// 1 + tanh cancels for negative x, and cost more.
+// `fast`: the result is kept in 16 bits.  silu and gelu are the tanh forms at every width, so that a gated pair has the same bits
+// whichever kernel computes it.
 template <int ACT>
 __device__ __forceinline__ float glu_of(float g, float u, float limit, bool fast) {
   if (ACT == GLU_CLAMP) {
     g = fminf(g, limit);
     const float b = fminf(fmaxf(u, -limit), limit) + 1.f;
     return (fast ? __fdividef(g, 1.0f + __expf(-1.702f * g)) : g / (1.0f + expf(-1.702f * g))) * b;
-  }
-  if (fast) {
-    const float z = ACT == GLU_GELU ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : g;
-    return __fdividef(g, 1.0f + __expf(-z)) * u;
   }
   return (ACT == GLU_GELU ? gelu_tanh(g) : silu_ref(g)) * u;
 }
