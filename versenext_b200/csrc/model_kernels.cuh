@@ -88,20 +88,18 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
   __shared__ float sm[8];
   const long long src = (long long)blockIdx.x * row_mul + row_add;   // e.g. the last position of every sequence
   const float* xr = x + src * D;
-  // rows of up to 4096 values on 16-byte boundaries stay in registers: one read, four values a load (4096 rows of 1024 took 9 us
-  // with a scalar read for the sum and another for the result)
-  const bool vec = D <= 4096 && (D & 3) == 0 && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)y32) & 15) == 0;
-  float4 v[4];
+  // rows of up to 4096 values stay in registers between the sum and the result: all loads in flight, one read
+  const bool held = D <= 4096;
+  float v[16];
   float ss = 0.f;
-  if (vec) {
+  if (held) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int d = (threadIdx.x + u * 256) * 4;
-      if (d < D) v[u] = load4(xr + d);
+    for (int u = 0; u < 16; ++u) {
+      const int d = threadIdx.x + u * 256;
+      v[u] = d < D ? xr[d] : 0.f;
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if ((threadIdx.x + u * 256) * 4 < D) ss += v[u].x * v[u].x + v[u].y * v[u].y + v[u].z * v[u].z + v[u].w * v[u].w;
+    for (int u = 0; u < 16; ++u) ss += v[u] * v[u];
   } else {
     for (int d = threadIdx.x; d < D; d += 256) ss += xr[d] * xr[d];
   }
@@ -113,14 +111,14 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
 #pragma unroll
   for (int i = 0; i < 8; ++i) tot += sm[i];
   const float r = sqrtf(tot / (float)D + eps);
-  if (vec) {
+  if (held) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int d = (threadIdx.x + u * 256) * 4;
+    for (int u = 0; u < 16; ++u) {
+      const int d = threadIdx.x + u * 256;
       if (d >= D) break;
-      const float4 f = load4(w + d), o = make_float4(v[u].x / r * f.x, v[u].y / r * f.y, v[u].z / r * f.z, v[u].w / r * f.w);
-      if (y) store4(y + (long long)blockIdx.x * D + d, o);
-      if (y32) store4(y32 + (long long)blockIdx.x * D + d, o);
+      const float o = v[u] / r * w[d];
+      if (y) y[(long long)blockIdx.x * D + d] = from_f<T>(o);
+      if (y32) y32[(long long)blockIdx.x * D + d] = o;
     }
     return;
   }
