@@ -76,3 +76,26 @@ def test_three_path_attention(n_head, n_kv, dim, window, n_sink, alibi, ctx, new
     got = m.forward_cached(toks[:, ctx:], cache, parents=parents).numpy()
     want, _ = OM.forward(sd, cfg, toks[:, ctx:], cache=oc, parents=parents)
     assert np.max(np.abs(got - want)) / np.max(np.abs(want)) < 1e-4      # float32 on both sides, sums in other orders
+
+
+@pytest.mark.parametrize("n_head,n_kv,dim,window,B,T", [(4, 4, 64, 8, 1, 40), (4, 2, 256, 5, 2, 300), (2, 1, 32, 3, 40, 12)])
+def test_a_value_that_is_no_number_stays_in_its_window(n_head, n_kv, dim, window, B, T):
+    """A token whose embedding is NaN puts NaN into the keys and values of its position.  Rows whose window ends before it are what they
+    are with any other token there, although their block's neighbours see the position."""
+    from oracle import model as OM
+    cfg = OM.small_config(vocab_size=50, dim=dim, n_layer=1, n_head=n_head, n_kv_head=n_kv, window_size=window, num_global_tokens=2,
+                          use_alibi=False, use_rope=True, max_seq_len=512, init_std=0.2)
+    sd = OM.init_state_dict(cfg, seed=5, gate_std=1.0)
+    sd["tok_emb.weight"] = sd["head.weight"] = sd["tok_emb.weight"].copy()
+    sd["tok_emb.weight"][49] = np.nan
+    kw = cfg.to_dict()
+    kw.pop("init_std")
+    m = vn.VerseNexLM(dtype="f32", **kw)
+    m.load_state_dict(sd)
+    toks = np.random.default_rng(1).integers(0, 49, (B, T))
+    got = []
+    for first in (7, 49):
+        toks[:, 0] = first
+        got.append(m.forward_cached(toks, m.new_cache(B, T), want_logits=False, want_hidden=True).numpy())
+    assert np.all(np.isnan(got[1][:, :window])) and np.all(np.isfinite(got[0]))
+    np.testing.assert_array_equal(got[0][:, window:], got[1][:, window:])

@@ -201,12 +201,13 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             : "=r"(go) : "r"(mine) : "memory");
       }
       if (!go) break;
-      const int nchunk = (cnt + 31) >> 5;
+      // chunk_no counts staged chunks only: the wait before a tensor store lets the last one read on, so the next has to take the
+      // other staging tile, whatever was left out in between
+      const int nchunk = n0 < g.N ? (cnt + 31) >> 5 : 0;   // the pair's second CTA may have no features
       for (int ch = grp; ch < nchunk; ch += 2, ++chunk_no) {
         unsigned r[32];
         tmem_ld32(tmem_base + (unsigned)buf * 256u + ((unsigned)(q * 32) << 16) + (unsigned)(ch * 32), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (n0 >= g.N) continue;                        // uniform: the pair's second CTA may have no features
         if (MODE == TC_SWIGLU && g.c_bf16) {
           pair_glu_chunk(g, r, ch, q, lane, n0, row0, cnt);
         } else if (MODE == TC_STORE && g.tma_out && ch * 32 + 32 <= cnt) {

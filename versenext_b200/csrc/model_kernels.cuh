@@ -566,9 +566,10 @@ __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, 
     const float ga = la > 0.f ? a.g_a / la : 0.f, gb = lb > 0.f ? a.g_b / lb : 0.f, gc = lc > 0.f ? a.g_c / lc : 0.f;
     for (int j = lane; j < nk; j += 32) {
       const int dist = distance(j);
-      float w = dist < 0 ? -1.f : 0.f;                   // below zero: not this row's key, whatever its value is
-      if (dist >= 0 && dist < a.window) w = ga * expf(row[j] - ma);
-      if (dist >= 0 && use_c && (a.alibi_window == 0 || dist < a.alibi_window)) w += gc * expf(row[j] - slope * (float)dist - mc);
+      const bool in_a = dist >= 0 && dist < a.window, in_c = dist >= 0 && use_c && (a.alibi_window == 0 || dist < a.alibi_window);
+      float w = in_a || in_c ? 0.f : -1.f;               // below zero: no path of this row takes the key, whatever its value is
+      if (in_a) w = ga * expf(row[j] - ma);
+      if (in_c) w += gc * expf(row[j] - slope * (float)dist - mc);
       row[j] = w;
     }
     for (int j = nk + lane; j < total; j += 32) row[j] = gb * expf(row[j] - mb);
