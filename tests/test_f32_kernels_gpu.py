@@ -99,3 +99,31 @@ def test_a_value_that_is_no_number_stays_in_its_window(n_head, n_kv, dim, window
         got.append(m.forward_cached(toks, m.new_cache(B, T), want_logits=False, want_hidden=True).numpy())
     assert np.all(np.isnan(got[1][:, :window])) and np.all(np.isfinite(got[0]))
     np.testing.assert_array_equal(got[0][:, window:], got[1][:, window:])
+
+
+def test_threads_launch_two_sizes():
+    """One context per thread: the shared memory that a kernel may ask for belongs to the function, so a smaller launch of one thread must
+    not take away what a larger one of the other is about to use."""
+    import threading
+    be, rng, results = vn.get_backend("cuda"), np.random.default_rng(3), {}
+
+    def run(Tk, q, k, v):
+        ctx = vn.Context(0)
+        try:
+            d = [ctx.from_numpy(a) for a in (q, k, v)]
+            out = ctx.empty(q.shape, np.float32)
+            for _ in range(4000):
+                ctx._check(ctx.lib.vn_attention(ctx.handle, *(a.ptr for a in d), None, out.ptr, 1, 2, Tk, 4))
+            results[Tk] = out.numpy()
+        except RuntimeError as e:
+            results[Tk] = e
+
+    inputs = {Tk: [rng.standard_normal((1, n, 4)).astype(np.float32) for n in (2, Tk, Tk)] for Tk in (12800, 12100)}
+    threads = [threading.Thread(target=run, args=(Tk, *a)) for Tk, a in inputs.items()]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for Tk, a in inputs.items():
+        assert not isinstance(results[Tk], Exception), results[Tk]
+        np.testing.assert_array_equal(results[Tk], be.attention(*a).numpy())

@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(256) trisparse_attn_kernel(AttnArgs a) {
 // each score is replaced by the sum of its gated probabilities; (3) S times the values, tile by tile.  Bound by latency: small
 // models have few rows and a warp that walks the keys alone (the kernel above) spends its time in a chain of exponentials,
 // 8 to 20 us a layer where this one takes 4 to 9 (float32, 64 wide heads, 5 rows at context 32, 2 x 300 rows of prompts).
-constexpr int TR_TILE = 64, TR_THREADS = 128;
+constexpr int TR_TILE = 64, TR_THREADS = 128, TR_SMEM = 160 * 1024;
 // FRESH: AttnArgs::fresh, apart because the code for it costs the prompts 2 % (282 -> 288 us for 2 x 300 rows)
 template <typename T, int R, bool FRESH>
 __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, int cap) {
@@ -614,7 +614,7 @@ inline TrisparsePlan trisparse_plan(const vn_ctx* ctx, const AttnArgs& a, int B)
   if (a.use_alibi && a.alibi_window == 0) keys = std::max(keys, std::min<long long>(a.max_seq, (long long)a.alibi_max + grown));
   const long long cap = (keys + a.n_sink) | 1;
   const long long smem = (TR_TILE * (a.hd + 4) + R * a.hd + R * cap) * 4;
-  return {R, cap, smem, smem <= 160 * 1024 && B <= 65535 && a.n_kv <= 65535};
+  return {R, cap, smem, smem <= TR_SMEM && B <= 65535 && a.n_kv <= 65535};
 }
 
 // The rows kernel where a block's scores fit shared memory, else the one-warp-per-row kernel (windows of many thousand keys).
@@ -629,8 +629,14 @@ inline int32_t launch_trisparse(vn_ctx* ctx, const AttnArgs& a, int B) {
     return VN_OK;
   }
   dim3 grid(ceil_div(n_items, R), a.n_kv, B);
+  // the limit belongs to the function on its device, whatever context or thread launches it: set once, to the most a plan admits
+  static unsigned long long attr_set = 0;
+  if (!((attr_set >> (ctx->device & 63)) & 1ull)) {
+    for (auto kernel : {trisparse_rows_kernel<T, 4, false>, trisparse_rows_kernel<T, 4, true>, trisparse_rows_kernel<T, 8, false>, trisparse_rows_kernel<T, 8, true>})
+      VN_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TR_SMEM));
+    attr_set |= 1ull << (ctx->device & 63);
+  }
   auto launch = [&](auto kernel) -> int32_t {
-    if (smem > 48 * 1024) VN_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     VN_LAUNCH_NAMED(ctx, "trisparse_rows_kernel", kernel, grid, TR_THREADS, smem, a, (int)cap);
     return VN_OK;
   };

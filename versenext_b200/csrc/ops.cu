@@ -152,6 +152,9 @@ __global__ void __launch_bounds__(256) attention_row_kernel(const float* __restr
   }
 }
 
+constexpr int64_t AT_MAX_TK = 12800;
+constexpr size_t attention_row_smem(int64_t Tk) { return (size_t)((Tk + 3) & ~(int64_t)3) * sizeof(float) + 256 * sizeof(float4); }
+
 // Tiles of 64 queries x 64 keys, heads of up to DM.  A warp owns 16 query rows; its 16 lanes of a row hold the row's scores of four
 // keys each, so that the online soft-max needs shuffles only, and DM / 16 of its results.  Per thread 8 x 4 products of
 // float4s along the head (12 shared loads for 128 FMAs) for the scores, 8 x DM / 16 along the keys for the values: the
@@ -395,7 +398,8 @@ int32_t vn_attention(vn_ctx* ctx, const float* q, const float* k, const float* v
   VN_REQUIRE(ctx, q && k && v && out && BH >= 0 && Tq >= 0 && Tk >= 1 && D >= 1, "bad arguments");
   VN_REQUIRE(ctx, BH < 65536, "too many batch*heads");
   if (BH * Tq == 0) return VN_OK;
-  VN_REQUIRE(ctx, (size_t)4 * Tk * sizeof(float) <= 200 * 1024, "Tk %lld too long for the backend attention op", (long long)Tk);
+  // one limit for every shape, whichever kernel takes it (the row kernel keeps a row of scores in shared memory, the tile kernel none)
+  VN_REQUIRE(ctx, Tk <= AT_MAX_TK, "Tk %lld too long for the backend attention op", (long long)Tk);
   const int vec = D % 4 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0;
   const float scale = 1.0f / sqrtf((float)D);
   // A tile's 64 rows share the keys that are loaded; below a quarter of them a block per row is as fast and spreads over more SMs.
@@ -406,9 +410,13 @@ int32_t vn_attention(vn_ctx* ctx, const float* q, const float* k, const float* v
   }
   int lpk = 1;
   while (lpk < 32 && lpk * 4 < D) lpk *= 2;
-  const size_t smem = (size_t)((Tk + 3) & ~(int64_t)3) * sizeof(float) + 256 * sizeof(float4);
-  if (smem > 48 * 1024)
-    VN_CUDA(ctx, cudaFuncSetAttribute(attention_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the function's limit is shared by all contexts and threads on a device: set once, to the longest row
+  static unsigned long long attr_set = 0;
+  if (!((attr_set >> (ctx->device & 63)) & 1ull)) {
+    VN_CUDA(ctx, cudaFuncSetAttribute(attention_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attention_row_smem(AT_MAX_TK)));
+    attr_set |= 1ull << (ctx->device & 63);
+  }
+  const size_t smem = attention_row_smem(Tk);
   VN_REQUIRE(ctx, Tq < (1ll << 31), "too many queries");
   dim3 grid((unsigned)Tq, (unsigned)BH);
   VN_LAUNCH(ctx, attention_row_kernel, grid, 256, smem, q, k, v, mask, out, (long long)Tq, (int)Tk, (int)D, scale, lpk, vec);
