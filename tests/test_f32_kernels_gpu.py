@@ -127,3 +127,13 @@ def test_threads_launch_two_sizes():
     for Tk, a in inputs.items():
         assert not isinstance(results[Tk], Exception), results[Tk]
         np.testing.assert_array_equal(results[Tk], be.attention(*a).numpy())
+
+
+@pytest.mark.parametrize("Tq,D", [(2, 8), (2, 200), (20, 30), (70, 64), (65, 128)])
+def test_attention_of_values_near_the_largest(Tq, D):
+    """A weighted mean is no larger than what it is taken of: values of 3e38 over hundreds of keys stay finite."""
+    rng = np.random.default_rng(Tq + D)
+    q, k = (rng.standard_normal((2, n, D)).astype(np.float32) for n in (Tq, 500))
+    v = (3e38 * np.sign(rng.standard_normal(D)) * np.ones((2, 500, D))).astype(np.float32)
+    got = vn.get_backend("cuda").attention(q, k, v).numpy().astype(np.float64)
+    assert np.all(np.abs(got / v[:, :1].astype(np.float64) - 1) <= (500 + 8 * 8 + 8) * EPS)   # 500 weights, eight tiles' rescaling

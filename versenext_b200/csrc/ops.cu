@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(256) attention_row_kernel(const float* __restr
   float l = 0.f;
   for (int j = tid; j < Tk; j += 256) { const float e = expf(sc[j] - m); sc[j] = e; l += e; }
   l = block_reduce<256>(l, false, red);
+  for (int j = tid; j < Tk; j += 256) sc[j] /= l;    // before the values: their weighted mean fits wherever they do
   __syncthreads();
   for (int d0 = 0; d0 < D; d0 += lpk * 4) {
     const int d = d0 + li * 4;
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(256) attention_row_kernel(const float* __restr
       if (d0 + e < D) {
         float s = 0.f;
         for (int gi = 0; gi < ng; ++gi) s += reinterpret_cast<const float*>(part)[gi * lpk * 4 + e];
-        out[(bh * Tq + qi) * D + d0 + e] = s / l;
+        out[(bh * Tq + qi) * D + d0 + e] = s;
       }
     }
     __syncthreads();
@@ -249,24 +250,27 @@ __global__ void __launch_bounds__(128) attention_tile_kernel(const float* __rest
       }
 #pragma unroll
       for (int x = 8; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
-      // nothing but -inf so far: exponentials of -inf are then zero, and a row of nothing else ends as 0 / 0
+      // nothing but -inf so far: exponentials of -inf are then zero, and a row of nothing else ends without a sum
       const float at = top == -CUDART_INF_F ? 0.f : top;
       const float fade = expf(m[i] - at);
       float sum = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float e = expf(s[j] - at);
-        sP[(ty + 8 * i) * LDP + tx + 16 * j] = e;
-        sum += e;
+        s[j] = expf(s[j] - at);
+        sum += s[j];
       }
 #pragma unroll
       for (int x = 8; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
-      l[i] = l[i] * fade + sum;
+      // the results so far stay weighted means of values (their sum would leave fp32 where the mean does not)
+      const float all = l[i] * fade + sum, inv = all == 0.f ? 0.f : 1.f / all, keep = l[i] * fade * inv;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sP[(ty + 8 * i) * LDP + tx + 16 * j] = s[j] * inv;
+      l[i] = all;
       m[i] = top;
 #pragma unroll
       for (int c = 0; c < DC / 2; ++c) {
         const float2 t = unpack2(o[i][c]);
-        o[i][c] = pack2(t.x * fade, t.y * fade);
+        o[i][c] = pack2(t.x * keep, t.y * keep);
       }
     }
     asm volatile("cp.async.wait_group 0;");          // the values are there
@@ -309,8 +313,8 @@ __global__ void __launch_bounds__(128) attention_tile_kernel(const float* __rest
     for (int c = 0; c < DC / 2; ++c) {
       const int d = DC < 4 ? tx * 2 : tx * 4 + (c >> 1) * 64 + (c & 1) * 2;
       const float2 t = unpack2(o[i][c]);
-      if (d < D) out[(bh * Tq + row) * D + d] = t.x / l[i];
-      if (d + 1 < D) out[(bh * Tq + row) * D + d + 1] = t.y / l[i];
+      if (d < D) out[(bh * Tq + row) * D + d] = l[i] == 0.f ? CUDART_NAN_F : t.x;
+      if (d + 1 < D) out[(bh * Tq + row) * D + d + 1] = l[i] == 0.f ? CUDART_NAN_F : t.y;
     }
   }
 }
