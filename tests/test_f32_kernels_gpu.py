@@ -137,3 +137,32 @@ def test_attention_of_values_near_the_largest(Tq, D):
     v = (3e38 * np.sign(rng.standard_normal(D)) * np.ones((2, 500, D))).astype(np.float32)
     got = vn.get_backend("cuda").attention(q, k, v).numpy().astype(np.float64)
     assert np.all(np.abs(got / v[:, :1].astype(np.float64) - 1) <= (500 + 8 * 8 + 8) * EPS)   # 500 weights, eight tiles' rescaling
+
+
+# window and cache of thousands of keys, short contexts (the kernel is chosen by what a block may see): few blocks of one SM each, blocks that
+# share SMs, more blocks than the SMs hold at once, scores beyond shared memory
+@pytest.mark.parametrize("window,B,T,ctx,kernel", [(9000, 1, 5, 30, "rows"), (9000, 2, 200, 0, "attn"), (10000, 1, 5, 30, "attn"), (10000, 2, 40, 7, "attn"),
+                                                   (4000, 2, 200, 0, "rows"), (6000, 2, 200, 3, "attn"), (3000, 8, 100, 0, "rows"), (40, 64, 5, 9, "rows")])
+@pytest.mark.parametrize("alibi", [False, True])
+def test_wide_windows(window, B, T, ctx, kernel, alibi):
+    from oracle import model as OM
+    cfg = OM.small_config(vocab_size=50, dim=64, n_layer=1, n_head=4, n_kv_head=2, window_size=window, num_global_tokens=3, use_alibi=alibi,
+                          use_rope=not alibi, max_seq_len=window + 100, init_std=0.2)
+    sd = OM.init_state_dict(cfg, seed=5, gate_std=1.0)
+    kw = cfg.to_dict()
+    kw.pop("init_std")
+    m = vn.VerseNexLM(dtype="f32", **kw)
+    m.load_state_dict(sd)
+    toks = np.random.default_rng(1).integers(0, 50, (B, ctx + T))
+    cache, oc = m.new_cache(B, window + 100), None
+    if ctx:
+        m.forward_cached(toks[:, :ctx], cache, last_only=True)
+        cache.commit(ctx, np.full(B, ctx, np.int32))
+        _, oc = OM.forward(sd, cfg, toks[:, :ctx])
+    m.ctx.profile(True)
+    got = m.forward_cached(toks[:, ctx:], cache).numpy()
+    ran = m.ctx.profile_report()
+    m.ctx.profile(False)
+    assert any(f"trisparse_{kernel}_kernel" in name for name in ran), list(ran)
+    want, _ = OM.forward(sd, cfg, toks[:, ctx:], cache=oc)
+    assert np.max(np.abs(got - want)) / np.max(np.abs(want)) < 1e-4      # float32 on both sides, sums in other orders

@@ -603,21 +603,37 @@ __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, 
   }
 }
 
-struct TrisparsePlan { int R; long long cap, smem; bool rows; };
+struct TrisparsePlan { int R; long long cap, smem, blocks, per_sm; bool rows; };
+// Rows kernel or the one-warp kernel, and rows of a block.  A block's time goes with the keys it may see and hardly with its rows, so
+// eight rows pay once they fill the SMs one and a half times over (5 rows of 64 sequences, 4 heads, window 300: 68 us with four, 50 with
+// eight; 300 rows of one sequence: 44 and 54).  Scores take shared memory with the window: with three blocks or more on an SM
+// the rows kernel is the faster one (4 x 300 rows, 4 heads of 64, window 2000: 467 us against 555), with fewer only while the grid
+// is on the SMs at once (window 4000: 5 rows of 32 sequences 290 against 1060, 300 rows of one 545 against 493, 4 x 300 1329 against 1060;
+// window 9000, 300 rows: 1543 against 1071).  Four rows, three blocks: up to six rounds (8 heads, window 3000: 4 x 300 1316 against
+// 1682, 4 x 900 3726 against 3572).
 inline TrisparsePlan trisparse_plan(const vn_ctx* ctx, const AttnArgs& a, int B) {
   const int n_rep = a.H / a.n_kv, n_items = a.Tn * n_rep;
-  // eight rows a block once that gives two blocks per SM, four (shorter soft-maxes per warp) before
-  const int R = (long long)ceil_div(n_items, 8) * a.n_kv * B >= 2ll * ctx->sm_count ? 8 : 4;
-  // keys a block may see: all of them while path C is on (at most alibi_max, and a tree's nodes), else a window
-  const long long grown = a.anc ? a.Tn : R;
-  long long keys = std::min<long long>(a.max_seq, (long long)std::max(a.window, a.alibi_window) + grown);
-  if (a.use_alibi && a.alibi_window == 0) keys = std::max(keys, std::min<long long>(a.max_seq, (long long)a.alibi_max + grown));
-  const long long cap = (keys + a.n_sink) | 1;
-  const long long smem = (TR_TILE * (a.hd + 4) + R * a.hd + R * cap) * 4;
-  return {R, cap, smem, smem <= TR_SMEM && B <= 65535 && a.n_kv <= 65535};
+  const long long sm = ctx->sm_count;
+  auto plan = [&](int R) {
+    // keys a block may see: all of them while path C is on (at most alibi_max, and a tree's nodes), else a window
+    const long long grown = a.anc ? a.Tn : R;
+    long long keys = std::min<long long>(a.max_seq, (long long)std::max(a.window, a.alibi_window) + grown);
+    if (a.use_alibi && a.alibi_window == 0) keys = std::max(keys, std::min<long long>(a.max_seq, (long long)a.alibi_max + grown));
+    TrisparsePlan p;
+    p.R = R; p.cap = (keys + a.n_sink) | 1;
+    p.smem = (TR_TILE * (a.hd + 4) + R * a.hd + R * p.cap) * 4;
+    p.blocks = (long long)ceil_div(n_items, R) * a.n_kv * B;
+    p.per_sm = 228 * 1024 / (p.smem + 1024);
+    return p;
+  };
+  TrisparsePlan p = plan(8);
+  if (2 * p.blocks < 3 * sm || p.per_sm < 3) p = plan(4);
+  const long long once = p.per_sm * sm;
+  p.rows = p.smem <= TR_SMEM && B <= 65535 && a.n_kv <= 65535 &&
+           (p.blocks <= once || p.per_sm >= 4 || (p.per_sm == 3 && (p.R == 8 || p.blocks <= 6 * once)));
+  return p;
 }
 
-// The rows kernel where a block's scores fit shared memory, else the one-warp-per-row kernel (windows of many thousand keys).
 template <typename T>
 inline int32_t launch_trisparse(vn_ctx* ctx, const AttnArgs& a, int B) {
   const TrisparsePlan p = trisparse_plan(ctx, a, B);
