@@ -171,7 +171,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
           __syncwarp();
           if (++s == P2_STAGES) { s = 0; ph ^= 1u; }
         }
-        if (elect_one()) umma_commit_pair(&acc_full[buf]);
+        if (ok && elect_one()) umma_commit_pair(&acc_full[buf]);   // an unfinished tile is nobody's: both CTAs' epilogues give up
         __syncwarp();
         ++t;
       }
