@@ -303,14 +303,33 @@ inline int32_t launch_gemm_tc2(vn_ctx* ctx, const GemmArgs& g, long long a_rows_
   return VN_OK;
 }
 
-// Many rows, either kernel.  The pair kernel takes over where its 256 x 256 tiles fill the SM pairs: twice over for stores and gated
-// pairs (2528 x 4096 x 1024 32 -> 29 us, 1024 x 32000 x 1024 85 -> 71; 4096 x 2048 x 1024, not quite two rounds, 21 against
-// 22), and from 12 tiles on where it adds to the residual, which costs the other kernel most (4096 x 1024 x 2752 45 -> 27,
-// 1024 x 1024 x 1024 20 -> 13).  Rows in tiles of 128 where those of 256 leave half of the pairs idle.
+// Whether the pair kernel ends before the one-SM kernel, which takes segments of g.M rows.  Both kernels' time goes in rounds over the
+// SMs.  A round of the one-SM kernel with segments of 32, 64 or 128 rows takes about 0.52, 0.58 or 0.7 of one with 256 rows.  The
+// pair kernel's round takes as long as that of 256 rows for stores and gated pairs (its last half tile of 128 features counts
+// whole: 8192 x 1152 x 1024, three rounds against two, 28 us against 19), 0.85 of it where it adds to the residual, which costs
+// the other kernel most, and 0.7 in tiles of 128 rows.  Measured over 12 widths, K of 64 to 2752 and 257 to 8192 rows: the kernel
+// chosen here was never more than 5 % the slower one.
+//  - Two rounds of pairs for stores and gated pairs, and 384 rows: 300 x 32000 x 512 stored 21.4 against 23.0 us.  From 12 tiles where it adds.
+//  - K: of short products the pair kernel's start and its write-out are the longer ones (one-SM against pair, 2048 rows x 8192).  Stored in
+//    32 bits, K = 128 19.3 against 22.6 us, K = 512 26.7 against 26.2; gated, K = 192 25.0 against 25.9, K = 256 25.8 against 26.0, 1024
+//    38 against 36; stored in 16 bits, K = 512 29.3 against 33.6, K = 1024 38.9 against 38.8; added, 2048 x 1152, K = 192 10.0
+//    against 10.9, K = 256 11.0 against 11.1, K = 512 14.1 against 12.5.
+// Experts' rows: the pieces that must exist, not those that may.
+inline bool gemm_tc2_pays(const vn_ctx* ctx, const GemmArgs& g, long long rows) {
+  using namespace tc_detail;
+  const bool add = g.epi == EPI_ADD;
+  const long long sm = ctx->sm_count, pairs = sm / 2, pieces = ceil_div(rows, 256ll), tiles = ceil_div(g.N, 2 * BF) * pieces;
+  if (g.K < (add || g.epi == EPI_SWIGLU ? 256 : g.c_bf16 ? 1024 : 512) || tiles < (add ? 12 : 2 * pairs) || (!add && rows <= 384)) return false;
+  const double one = (double)ceil_div(ceil_div(g.N, BF) * (g.seg_cnt ? pieces : (long long)g.nseg), sm) * (g.M > 128 ? 1.0 : g.M > 64 ? 0.7 : g.M > 32 ? 0.58 : 0.52);
+  const double two = 2 * tiles <= pairs ? 0.7 : (double)ceil_div(tiles, pairs) * (add ? 0.85 : 1.0);
+  return two <= one;
+}
+
+// Many rows, either kernel.  Rows in tiles of 128 where those of 256 leave half of the pairs idle.
 inline int32_t launch_gemm_many(vn_ctx* ctx, const GemmArgs& g, long long a_rows_total, TcPlan& plan) {
-  const int pairs = ctx->sm_count / 2;
-  const long long tiles = (long long)ceil_div(g.N, 2 * tc_detail::BF) * (g.seg_cnt ? (long long)g.nseg : ceil_div(a_rows_total, 256ll));
-  if (gemm_tc2_supported(g) && tiles >= (g.epi == EPI_ADD ? 12 : 2 * pairs))
-    return launch_gemm_tc2(ctx, g, a_rows_total, 2 * tiles <= pairs ? 128 : 256, plan.error_flag);
+  if (gemm_tc2_supported(g) && gemm_tc2_pays(ctx, g, a_rows_total)) {
+    const long long tiles = ceil_div(g.N, 2 * tc_detail::BF) * ceil_div(a_rows_total, 256ll);
+    return launch_gemm_tc2(ctx, g, a_rows_total, 4 * tiles <= ctx->sm_count ? 128 : 256, plan.error_flag);
+  }
   return launch_gemm_tc(ctx, g, a_rows_total, plan);
 }
