@@ -156,6 +156,13 @@ __global__ void __launch_bounds__(256) attention_row_kernel(const float* __restr
 constexpr int64_t AT_MAX_TK = 12800;
 constexpr size_t attention_row_smem(int64_t Tk) { return (size_t)((Tk + 3) & ~(int64_t)3) * sizeof(float) + 256 * sizeof(float4); }
 
+// the power of two u with x u in [1/2, 1), for a sum x of exponentials (zero, or 1 to AT_MAX_TK); unit_of(x) / unit_of(from)
+__device__ __forceinline__ unsigned exponent_of(float x) { return __float_as_uint(x) & 0x7f800000u; }
+__device__ __forceinline__ float unit_of(float x) { return __uint_as_float((253u << 23) - exponent_of(x)); }
+__device__ __forceinline__ float unit_ratio(float x, float from) {
+  return __uint_as_float((127u << 23) + max(exponent_of(from), 64u << 23) - exponent_of(x));   // from zero: any finite value
+}
+
 // Tiles of 64 queries x 64 keys, heads of up to DM.  A warp owns 16 query rows; its 16 lanes of a row hold the row's scores of four
 // keys each, so that the online soft-max needs shuffles only, and DM / 16 of its results.  Per thread 8 x 4 products of
 // float4s along the head (12 shared loads for 128 FMAs) for the scores, 8 x DM / 16 along the keys for the values: the
@@ -261,10 +268,11 @@ __global__ void __launch_bounds__(128) attention_tile_kernel(const float* __rest
       }
 #pragma unroll
       for (int x = 8; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
-      // the results so far stay weighted means of values (their sum would leave fp32 where the mean does not)
-      const float all = l[i] * fade + sum, inv = all == 0.f ? 0.f : 1.f / all, keep = l[i] * fade * inv;
+      // weights in units of a power of two above their sum: sums of values stay within the values' range, and nothing is rounded for it
+      // (32 heads x 500 x 500 x 64: 80 us, with 1 / sum instead 85, with sums that may overflow 78).  Before the first key fade is zero.
+      const float all = l[i] * fade + sum, unit = unit_of(all), keep = fade * unit_ratio(all, l[i]);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) sP[(ty + 8 * i) * LDP + tx + 16 * j] = s[j] * inv;
+      for (int j = 0; j < 4; ++j) sP[(ty + 8 * i) * LDP + tx + 16 * j] = s[j] * unit;
       l[i] = all;
       m[i] = top;
 #pragma unroll
@@ -309,12 +317,13 @@ __global__ void __launch_bounds__(128) attention_tile_kernel(const float* __rest
   for (int i = 0; i < 8; ++i) {
     const long long row = q0 + ty + 8 * i;
     if (row >= Tq) continue;
+    const float all = l[i] * unit_of(l[i]);
 #pragma unroll
     for (int c = 0; c < DC / 2; ++c) {
       const int d = DC < 4 ? tx * 2 : tx * 4 + (c >> 1) * 64 + (c & 1) * 2;
       const float2 t = unpack2(o[i][c]);
-      if (d < D) out[(bh * Tq + row) * D + d] = l[i] == 0.f ? CUDART_NAN_F : t.x;
-      if (d + 1 < D) out[(bh * Tq + row) * D + d + 1] = l[i] == 0.f ? CUDART_NAN_F : t.y;
+      if (d < D) out[(bh * Tq + row) * D + d] = t.x / all;
+      if (d + 1 < D) out[(bh * Tq + row) * D + d + 1] = t.y / all;
     }
   }
 }
