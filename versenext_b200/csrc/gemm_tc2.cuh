@@ -305,9 +305,10 @@ inline int32_t launch_gemm_tc2(vn_ctx* ctx, const GemmArgs& g, long long a_rows_
 
 // Whether the pair kernel ends before the one-SM kernel, which takes segments of g.M rows.  Both kernels' time goes in rounds over the
 // SMs.  A round of the one-SM kernel with segments of 32, 64 or 128 rows takes about 0.52, 0.58 or 0.7 of one with 256 rows.  The
-// pair kernel's round takes as long as that of 256 rows for stores and gated pairs (its last half tile of 128 features counts
-// whole: 8192 x 1152 x 1024, three rounds against two, 28 us against 19), 0.85 of it where it adds to the residual, which costs
-// the other kernel most, and 0.7 in tiles of 128 rows.  Measured over 12 widths, K of 64 to 2752 and 257 to 8192 rows: the kernel
+// pair kernel's round takes 0.9 of that of 256 rows for stores and gated pairs (its last half tile of 128 features counts whole:
+// 8192 x 1152 x 1024, three rounds against two, 28 us against 19; 16384 x 5504 x 1024 gated, 20 against 19, 169 against 212),
+// 0.85 where it adds to the residual, which costs the other kernel most, and 0.7 in tiles of 128 rows.  Measured over 12 widths, K
+// of 64 to 2752 and 257 to 8192 rows: the kernel
 // chosen here was never more than 5 % the slower one.
 //  - Two rounds of pairs for stores and gated pairs, and 384 rows: 300 x 32000 x 512 stored 21.4 against 23.0 us.  From 12 tiles where it adds.
 //  - K: of short products the pair kernel's start and its write-out are the longer ones (one-SM against pair, 2048 rows x 8192).  Stored in
@@ -321,7 +322,7 @@ inline bool gemm_tc2_pays(const vn_ctx* ctx, const GemmArgs& g, long long rows) 
   const long long sm = ctx->sm_count, pairs = sm / 2, pieces = ceil_div(rows, 256ll), tiles = ceil_div(g.N, 2 * BF) * pieces;
   if (g.K < (add || g.epi == EPI_SWIGLU ? 256 : g.c_bf16 ? 1024 : 512) || tiles < (add ? 12 : 2 * pairs) || (!add && rows <= 384)) return false;
   const double one = (double)ceil_div(ceil_div(g.N, BF) * (g.seg_cnt ? pieces : (long long)g.nseg), sm) * (g.M > 128 ? 1.0 : g.M > 64 ? 0.7 : g.M > 32 ? 0.58 : 0.52);
-  const double two = 2 * tiles <= pairs ? 0.7 : (double)ceil_div(tiles, pairs) * (add ? 0.85 : 1.0);
+  const double two = 2 * tiles <= pairs ? 0.7 : (double)ceil_div(tiles, pairs) * (add ? 0.85 : 0.9);
   return two <= one;
 }
 
