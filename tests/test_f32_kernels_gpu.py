@@ -166,3 +166,11 @@ def test_wide_windows(window, B, T, ctx, kernel, alibi):
     assert any(f"trisparse_{kernel}_kernel" in name for name in ran), list(ran)
     want, _ = OM.forward(sd, cfg, toks[:, ctx:], cache=oc)
     assert np.max(np.abs(got - want)) / np.max(np.abs(want)) < 1e-4      # float32 on both sides, sums in other orders
+
+
+# few keys: a block or a warp per row, on both sides of 512 rows, of a warp's lanes and of eight rows a block
+@pytest.mark.parametrize("BH,Tq,Tk,D", [(1, 600, 1, 1), (2, 300, 8, 33), (3, 200, 32, 16), (5, 128, 16, 32), (600, 1, 8, 100), (1, 513, 5, 128), (64, 8, 32, 64),
+                                        (2, 16, 32, 128), (1, 512, 31, 30), (103, 5, 7, 3)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_attention_of_few_keys(BH, Tq, Tk, D, masked):
+    test_attention(BH, Tq, Tk, D, masked)

@@ -153,6 +153,39 @@ __global__ void __launch_bounds__(256) attention_row_kernel(const float* __restr
   }
 }
 
+// Few keys (at most a warp's lanes): a warp per query row, a lane per key, then a lane per result.  No shared memory and no barrier: the
+// tile kernel's loads, soft-max and write-out take 8 to 16 us for a single tile of keys.
+__global__ void __launch_bounds__(256) attention_warp_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                                                             const float* __restrict__ mask, float* __restrict__ out, long long Tq, int Tk, int D,
+                                                             float scale, int vec) {
+  const int lane = threadIdx.x & 31;
+  const long long qi = (long long)blockIdx.x * 8 + (threadIdx.x >> 5), bh = blockIdx.y;
+  if (qi >= Tq) return;
+  const float* qr = q + (bh * Tq + qi) * D;
+  const float* kr = k + (bh * Tk + min(lane, Tk - 1)) * D;
+  const float* vb = v + bh * Tk * D;
+  float s = 0.f;
+  for (int d = 0; d < D; d += 4) {
+    const float4 a = row4(qr, d, D, vec), b = row4(kr, d, D, vec);
+    s = fmaf(a.x, b.x, s); s = fmaf(a.y, b.y, s); s = fmaf(a.z, b.z, s); s = fmaf(a.w, b.w, s);
+  }
+  s *= scale;
+  if (mask && lane < Tk) s += mask[qi * Tk + lane];
+  const float m = warp_max(lane < Tk ? s : -CUDART_INF_F);
+  const float e = lane < Tk ? expf(s - m) : 0.f;
+  const float p = e / warp_sumf(e);
+  for (int d0 = 0; d0 < D; d0 += 32) {
+    const int d = d0 + lane;
+    float acc = 0.f;
+#pragma unroll 8
+    for (int j = 0; j < Tk; ++j) {
+      const float w = __shfl_sync(0xffffffffu, p, j);
+      if (d < D) acc = fmaf(w, vb[(long long)j * D + d], acc);
+    }
+    if (d < D) out[(bh * Tq + qi) * D + d] = acc;
+  }
+}
+
 constexpr int64_t AT_MAX_TK = 12800;
 constexpr size_t attention_row_smem(int64_t Tk) { return (size_t)((Tk + 3) & ~(int64_t)3) * sizeof(float) + 256 * sizeof(float4); }
 
@@ -410,13 +443,23 @@ int32_t vn_attention(vn_ctx* ctx, const float* q, const float* k, const float* v
   VN_CHECK_CTX(ctx);
   VN_REQUIRE(ctx, q && k && v && out && BH >= 0 && Tq >= 0 && Tk >= 1 && D >= 1, "bad arguments");
   VN_REQUIRE(ctx, BH < 65536, "too many batch*heads");
+  VN_REQUIRE(ctx, Tq < (1ll << 31), "too many queries");
   if (BH * Tq == 0) return VN_OK;
   // one limit for every shape, whichever kernel takes it (the row kernel keeps a row of scores in shared memory, the tile kernel none)
   VN_REQUIRE(ctx, Tk <= AT_MAX_TK, "Tk %lld too long for the backend attention op", (long long)Tk);
   const int vec = D % 4 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0;
   const float scale = 1.0f / sqrtf((float)D);
   // A tile's 64 rows share the keys that are loaded; below a quarter of them a block per row is as fast and spreads over more SMs.
-  if (Tq >= 16 && D <= 128) {
+  // A tile of few keys is mostly fixed cost, 8 us for D of 32, 10 for 64, 16 for 128: a block per row up to 512 rows (16 x 8 keys x 64:
+  // 10.3 -> 4.6 us), a warp per row beyond (64 x 64 rows, D = 16, 4 keys: 8.3 -> 4.7; 512 x 4 rows: 10.3 -> 4.6 of blocks; at 512 products a
+  // row tiles are level, 64 x 128 rows x 16 keys x 32 8.3 against 12.4).
+  const bool few = Tk <= 32 && D <= 128, blocks = BH * Tq <= 512;
+  if (few && !blocks && (Tk <= 8 || Tk * D <= 512)) {
+    dim3 grid((unsigned)ceil_div(Tq, (int64_t)8), (unsigned)BH);
+    VN_LAUNCH(ctx, attention_warp_kernel, grid, 256, 0, q, k, v, mask, out, (long long)Tq, (int)Tk, (int)D, scale, vec);
+    return VN_OK;
+  }
+  if (Tq >= 16 && D <= 128 && !(few && blocks)) {
     if (D <= 32) return launch_attention_tile<32>(ctx, q, k, v, mask, out, BH, Tq, Tk, (int)D, scale, vec);
     if (D <= 64) return launch_attention_tile<64>(ctx, q, k, v, mask, out, BH, Tq, Tk, (int)D, scale, vec);
     return launch_attention_tile<128>(ctx, q, k, v, mask, out, BH, Tq, Tk, (int)D, scale, vec);
@@ -430,7 +473,6 @@ int32_t vn_attention(vn_ctx* ctx, const float* q, const float* k, const float* v
     attr_set |= 1ull << (ctx->device & 63);
   }
   const size_t smem = attention_row_smem(Tk);
-  VN_REQUIRE(ctx, Tq < (1ll << 31), "too many queries");
   dim3 grid((unsigned)Tq, (unsigned)BH);
   VN_LAUNCH(ctx, attention_row_kernel, grid, 256, smem, q, k, v, mask, out, (long long)Tq, (int)Tk, (int)D, scale, lpk, vec);
   return VN_OK;
