@@ -108,3 +108,10 @@ def test_half_k_blocks_on_pairs(monkeypatch):
     import bozasun_cases as C
     mlp = C.moe(experts=7, identity=3, top=3, groups=5, keep=2, ff=1024)
     assert _composed(C, [C.attention(mlp=mlp)], 5, 520, monkeypatch, {2}, width=264) < 2e-2
+
+
+def test_clamped_experts_on_pairs(monkeypatch):
+    """The clamped gated function on pairs, experts' inputs weighed first."""
+    import givozen_cases as C
+    mlp = C.moe(experts=7, top=3, ff=1024, shared_ff=64)
+    assert _composed(C, [C.attention(mlp=mlp)], 5, 520, monkeypatch, {2}, width=264) < 2e-2

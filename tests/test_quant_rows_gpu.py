@@ -58,3 +58,22 @@ def test_few_rows_of_a_wide_model(monkeypatch, scheme, B, T):
         got.append(m.forward_cached(toks[:, 7:], cache).numpy())
         m.check()
     assert np.linalg.norm(got[0] - got[1]) / np.linalg.norm(got[1]) < 4e-3     # as above
+
+
+@pytest.mark.parametrize("mod", [False, True])
+def test_switch_of_a_prompts_gemms(monkeypatch, mod):
+    """VN_PREFILL_TC=0 keeps a prompt's GEMMs on mma.sync, quantised or not; the last rows' head has few rows."""
+    from test_prompt_pairs_gpu import _kernels
+    cfg = OM.mate_config(vocab_size=131, dim=128, n_layer=1, n_head=2, n_kv_head=1, window_size=40, num_global_tokens=8, max_seq_len=300, init_std=0.05,
+                         num_dense_parts=2, num_experts_per_part=3, top_k=1, layer_pattern=["mod" if mod else "trisparse"])
+    kw = cfg.to_dict()
+    kw.pop("init_std")
+    m = vn.VerseNexLM(dtype="bf16", **kw)
+    m.load_state_dict(OM.init_state_dict(cfg, seed=3))
+    m.quantize("int8")
+    toks = m.ctx.from_numpy(np.random.default_rng(0).integers(0, 131, (3, 100)))
+    for flag in ("1", "0"):
+        monkeypatch.setenv("VN_PREFILL_TC", flag)
+        _, names = _kernels(lambda: m.forward_cached(toks, m.new_cache(3, 101)))
+        assert any("gemm_tcq_rows_kernel" in n for n in names) == (flag == "1"), names
+        assert any("gemm_mma_q_kernel" in n for n in names) == (flag == "0"), names

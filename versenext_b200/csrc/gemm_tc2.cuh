@@ -1,10 +1,10 @@
 // Dense GEMM of many rows (prompts) on pairs of SMs: tcgen05.mma with cta_group::2.
 //
 // The one-SM kernel of gemm_tc.cuh brings 48 KB into shared memory for 128 features x 256 rows of a k block and reads as much
-// again for the MMAs: 192 bytes a clock where shared memory gives 128, and 7.3 TB/s over all SMs where TMA delivers no more.
-// Here two CTAs of a cluster share a tile of 256 features x 256 rows: each loads its own 128 features and HALF of the rows,
-// the tensor cores of both read both halves, and the bytes per product fall by a third.  A k block takes 700 cycles (512 at the
-// MMA rate); 8192 x 2048 x 8192 385 -> 227 us (1213 TFLOP/s).
+// again for the MMAs: at the MMA rate 192 bytes a clock, where shared memory gives 128.  Here two CTAs of a cluster share a tile
+// of 256 features x 256 rows: each loads its own 128 features and HALF of the rows, the tensor cores of both read both halves,
+// and the bytes per product fall by a third.  8192 x 2048 x 8192 385 -> 227 us (1213 TFLOP/s); what TMA brings rises from 8.4 to
+// 9.5 TB/s over all SMs, most of it from L2, so neither kernel is at a fixed ceiling of that path.
 //
 // One cluster per SM pair walks the tiles (persistent); accumulators are double buffered in TMEM (2 x 256 columns), so a tile's
 // epilogue runs under the next tile's MMAs.  Per CTA: warp 0 TMA, warp 1 MMA (issued by the cluster's first CTA for both),

@@ -1,4 +1,5 @@
-// Weight-only quantised linears of many rows (prompts, large verification batches) on tcgen05.
+// Weight-only quantised linears on tcgen05, outside the split-K route of at most 256 rows (gemm_tcq.cuh): prompts, large verification
+// batches, the heads of prompts' last rows, and every row count of models wider than that route takes.
 //
 // As in gemm_tcq.cuh the weights travel as raw bytes and become the bf16 UMMA operand inside shared memory, here always as
 // the exact small integers.  A scale per output row is applied to the accumulator at the end; scales per 128 inputs (QMODE 3)
@@ -11,7 +12,9 @@
 // sums).  A converting warp has a stage of its own and takes every S-th k block, so that it sees each phase of its barrier in turn.
 // Bound by shared memory: a k block of 112 rows moves 70 KB through it (bytes in, operand out, both operands to the tensor
 // cores), 560 cycles at 128 bytes each, where its MMAs take 240 and a block was seen to take 700.  448 rows, INT4 groups / INT8:
-// 1024 -> 5504 28 / 26 us, -> 32,000 98 / 90 us; with mma.sync 61 us and 274 us for the groups.
+// 1024 -> 5504 28 / 26 us, -> 32,000 98 / 90 us; with mma.sync 61 us and 274 us for the groups.  Few rows leave SMs idle (no split along
+// K) and are still ahead of mma.sync: 1 / 32 / 128 rows of INT4 groups, 2560 -> 3584 27 / 27 / 29 us against 34 / 37 / 60, 6848 -> 2560
+// 57 / 58 / 62 against 85 / 93 / 150.
 #pragma once
 #include "gemm_tcq.cuh"
 

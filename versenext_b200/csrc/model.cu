@@ -385,9 +385,14 @@ int32_t ensure_partial(vn_model* m, size_t bytes);
 
 int32_t linear(vn_model* m, GemmArgs g) {
   vn_ctx* ctx = m->ctx;
+  // VN_PREFILL_TC=0 (read per call) keeps a prompt's GEMMs, those of more than 256 rows, on the mma.sync kernels
+  const char* pe = m->cfg.bf16 ? getenv("VN_PREFILL_TC") : nullptr;
+  const bool tc_rows = m->use_tc && !(g.M > 256 && pe && pe[0] == '0');
   if (g.wq) {
-    // dense blocks: the tensor-core kernel (VN_GEMM_TCQ=0 keeps mma.sync)
-    if (m->use_tc && !g.seg_cnt && gemm_tcq_rows_supported(g) && g.M <= 65535 * 64) {
+    // Dense blocks: the tensor-core kernel, at every row count (VN_GEMM_TCQ=0 keeps mma.sync).  Few rows come here from models wider than
+    // the split-K route's 2048 and from heads of prompts' last rows: 2560 wide, INT4, 1 to 64 rows against 13,696 features 25 to 31 us,
+    // mma.sync 50 to 56; 256 rows 50 and 136.
+    if (tc_rows && !g.seg_cnt && gemm_tcq_rows_supported(g) && g.M <= 65535 * 64) {
       TRY(ensure_partial(m, 1024));                               // the error word
       return launch_gemm_tcq_rows(ctx, g, g.M, m->tc_error);
     }
@@ -397,9 +402,8 @@ int32_t linear(vn_model* m, GemmArgs g) {
   if (m->cfg.bf16) {
     // Many rows (a prompt): the tcgen05 kernel takes the rows as segments of at most 256, every segment with the same
     // weight matrix.  A weight tile is then fetched once per segment, from L2 after the first.  Shorter segments where
-    // there would be fewer tiles than SMs.  VN_PREFILL_TC=0 (read per call) keeps the mma.sync kernel.
-    const char* pe = getenv("VN_PREFILL_TC");
-    if (m->use_tc && !(pe && pe[0] == '0') && g.M > 256 && !g.seg_cnt && !g.a_rows && g.nseg == 1 && (!g.bias || g.epi != EPI_SWIGLU) && !g.mul &&
+    // there would be fewer tiles than SMs.
+    if (tc_rows && g.M > 256 && !g.seg_cnt && !g.a_rows && g.nseg == 1 && (!g.bias || g.epi != EPI_SWIGLU) && !g.mul &&
         g.K % tc_detail::BK == 0 && g.N >= 16 && g.ldw_k == 1 && tc_detail::encode_fn() != nullptr &&
         (g.epi == EPI_STORE || g.epi == EPI_ADD || g.epi == EPI_SWIGLU) && (!g.post || g.c_bf16)) {
       TRY(ensure_partial(m, 1024));                               // the error word
