@@ -174,3 +174,9 @@ def test_wide_windows(window, B, T, ctx, kernel, alibi):
 @pytest.mark.parametrize("masked", [False, True])
 def test_attention_of_few_keys(BH, Tq, Tk, D, masked):
     test_attention(BH, Tq, Tk, D, masked)
+
+
+# matrices of many features: every number of rows that a pass takes, passes that are not full
+@pytest.mark.parametrize("M,N,K", [(1, 20001, 132), (2, 18944, 64), (3, 19003, 4), (4, 18945, 128), (7, 20011, 36), (8, 18950, 260), (17, 18947, 68), (32, 19001, 128)])
+def test_linears_of_many_features(M, N, K):
+    test_products("linear", M, N, K)

@@ -160,10 +160,13 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_f32_kernel(G
 // output each lane sums its k = 4 lane + 128 i terms in order (even and odd apart), then the lanes are added pair by pair; the NR x MR sums of a
 // warp are spread over its lanes while they are added (a lane passes on half of what it holds at each step), so that 32 sums
 // take 31 exchanges and every lane stores one of them.  NORM: every block normalises the few short rows of A into shared memory
-// for itself, a launch less on a chain that is nothing but launches.
+// for itself, a launch less on a chain that is nothing but launches.  MANY: matrices of many features, bound by HBM and so by the
+// weights that an SM has in flight: registers for two blocks of eight warps and more, rows addressed by 32-bit offsets.  Of few
+// features every SM has a few warps anyway, and these hold as much as they can (8 x 4096 x 1024: 7.2 us, with 128 registers 16).
+// 1 / 5 / 8 / 16 / 32 rows x 100,000 x 1024: 64 / 100 / 103 / 168 / 345 us, with one block of eight warps on an SM 68 / 160 / 160 / 239 / 418.
 constexpr int NR = 4, NORM_MAX = 4096;
-template <int MR, bool NORM>
-__global__ void __launch_bounds__(256, MR == 8 ? 1 : 2) gemm_f32_rows_kernel(GemmArgs g) {
+template <int MR, bool NORM, bool MANY>
+__global__ void __launch_bounds__(256, !MANY ? (MR == 8 ? 1 : 2) : MR == 1 ? 4 : MR == 2 ? 3 : 2) gemm_f32_rows_kernel(GemmArgs g) {
   const int lane = threadIdx.x & 31;
   const long long n0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * NR;
   const float* A = reinterpret_cast<const float*>(g.A);
@@ -195,6 +198,10 @@ __global__ void __launch_bounds__(256, MR == 8 ? 1 : 2) gemm_f32_rows_kernel(Gem
     f32x2 acc[NR * MR];
 #pragma unroll
     for (int i = 0; i < NR * MR; ++i) acc[i] = 0;
+    int off[MANY ? MR : 1];
+    if (MANY)
+#pragma unroll
+      for (int i = 0; i < MR; ++i) off[i] = (int)((m0 + i < g.M ? m0 + i : g.M - 1) * lda);
 #pragma unroll 1
     for (int k = lane * 4; k < g.K; k += 128) {
       ulonglong2 wv[NR];
@@ -203,7 +210,7 @@ __global__ void __launch_bounds__(256, MR == 8 ? 1 : 2) gemm_f32_rows_kernel(Gem
 #pragma unroll
       for (int i = 0; i < MR; ++i) {
         const int m = m0 + i < g.M ? m0 + i : g.M - 1;
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(A + m * lda + k);
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(MANY ? A + off[MANY ? i : 0] + k : A + m * lda + k);
 #pragma unroll
         for (int j = 0; j < NR; ++j) {
           fma2(acc[j * MR + i], x.x, wv[j].x);
@@ -254,8 +261,9 @@ inline int32_t launch_rows(vn_ctx* ctx, const GemmArgs& g) {
   // blocks of two warps while that leaves SMs without one, of eight where the matrix is large
   const int warps = g.N >= 8 * NR * 4 * ctx->sm_count ? 8 : 2;
   const char* name = g.tag ? g.tag : "gemm_f32_rows_kernel";
-  if (g.norm) VN_LAUNCH_NAMED(ctx, name, (gemm_f32_rows_kernel<MR, true>), ceil_div(g.N, warps * NR), warps * 32, 0, g);
-  else VN_LAUNCH_NAMED(ctx, name, (gemm_f32_rows_kernel<MR, false>), ceil_div(g.N, warps * NR), warps * 32, 0, g);
+  if (g.norm) VN_LAUNCH_NAMED(ctx, name, (gemm_f32_rows_kernel<MR, true, false>), ceil_div(g.N, warps * NR), warps * 32, 0, g);
+  else if (warps == 8 && g.M * g.lda < (1ll << 31)) VN_LAUNCH_NAMED(ctx, name, (gemm_f32_rows_kernel<MR, false, true>), ceil_div(g.N, warps * NR), warps * 32, 0, g);
+  else VN_LAUNCH_NAMED(ctx, name, (gemm_f32_rows_kernel<MR, false, false>), ceil_div(g.N, warps * NR), warps * 32, 0, g);
   return VN_OK;
 }
 
