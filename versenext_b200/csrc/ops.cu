@@ -4,7 +4,6 @@
 #include "gemm_f32.cuh"
 #include <math_constants.h>
 #include <stdint.h>
-#include <stdlib.h>
 
 namespace {
 using namespace f32_detail;
@@ -466,13 +465,13 @@ int32_t vn_attention(vn_ctx* ctx, const float* q, const float* k, const float* v
   }
   int lpk = 1;
   while (lpk < 32 && lpk * 4 < D) lpk *= 2;
-  // the function's limit is shared by all contexts and threads on a device: set once, to the longest row
+  const size_t smem = attention_row_smem(Tk);
+  // the function's limit is shared by all contexts and threads on a device: raised once, to the longest row
   static unsigned long long attr_set = 0;
-  if (!((attr_set >> (ctx->device & 63)) & 1ull)) {
+  if (smem > 48 * 1024 && !((attr_set >> (ctx->device & 63)) & 1ull)) {
     VN_CUDA(ctx, cudaFuncSetAttribute(attention_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attention_row_smem(AT_MAX_TK)));
     attr_set |= 1ull << (ctx->device & 63);
   }
-  const size_t smem = attention_row_smem(Tk);
   dim3 grid((unsigned)Tq, (unsigned)BH);
   VN_LAUNCH(ctx, attention_row_kernel, grid, 256, smem, q, k, v, mask, out, (long long)Tq, (int)Tk, (int)D, scale, lpk, vec);
   return VN_OK;
