@@ -613,7 +613,8 @@ __global__ void __launch_bounds__(TR_THREADS) trisparse_rows_kernel(AttnArgs a, 
 struct TrisparsePlan { int R; long long cap, smem, blocks, per_sm; bool rows; };
 // Rows kernel or the one-warp kernel, and rows of a block.  A block's time goes with the keys it may see and hardly with its rows, so
 // eight rows pay once they fill the SMs one and a half times over (5 rows of 64 sequences, 4 heads, window 300: 68 us with four, 50 with
-// eight; 300 rows of one sequence: 44 and 54).  Scores take shared memory with the window: with three blocks or more on an SM
+// eight; 300 rows of one sequence: 44 and 54) and a block has more than four (one token of 128 sequences, 4 heads of 64, context 600:
+// 143 us with eight, 118 with four).  Scores take shared memory with the window: with three blocks or more on an SM
 // the rows kernel is the faster one (4 x 300 rows, 4 heads of 64, window 2000: 467 us against 555), with fewer only while the grid
 // is on the SMs at once (window 4000: 5 rows of 32 sequences 290 against 1060, 300 rows of one 545 against 493, 4 x 300 1329 against 1060;
 // window 9000, 300 rows: 1543 against 1071).  Four rows, three blocks: up to six rounds (8 heads, window 3000: 4 x 300 1316 against
@@ -634,7 +635,7 @@ inline TrisparsePlan trisparse_plan(const vn_ctx* ctx, const AttnArgs& a, int B)
     return p;
   };
   TrisparsePlan p = plan(8);
-  if (2 * p.blocks < 3 * sm || p.per_sm < 3) p = plan(4);
+  if (n_items <= 4 || 2 * p.blocks < 3 * sm || p.per_sm < 3) p = plan(4);
   const long long once = p.per_sm * sm;
   p.rows = p.smem <= TR_SMEM && B <= 65535 && a.n_kv <= 65535 &&
            (p.blocks <= once || p.per_sm >= 4 || (p.per_sm == 3 && (p.R == 8 || p.blocks <= 6 * once)));
