@@ -180,3 +180,19 @@ def test_attention_of_few_keys(BH, Tq, Tk, D, masked):
 @pytest.mark.parametrize("M,N,K", [(1, 20001, 132), (2, 18944, 64), (3, 19003, 4), (4, 18945, 128), (7, 20011, 36), (8, 18950, 260), (17, 18947, 68), (32, 19001, 128)])
 def test_linears_of_many_features(M, N, K):
     test_products("linear", M, N, K)
+
+
+def test_wide_windows_of_many_rows():
+    """More rows than the one-warp kernel's grid has: the rows kernel, whatever is faster.  Every sequence alike, so that one is the answer."""
+    from oracle import model as OM
+    cfg = OM.small_config(vocab_size=50, dim=32, n_layer=1, n_head=1, n_kv_head=1, window_size=6000, num_global_tokens=3, use_alibi=False, use_rope=True,
+                          max_seq_len=6100, init_std=0.2)
+    sd = OM.init_state_dict(cfg, seed=5, gate_std=1.0)
+    kw = cfg.to_dict()
+    kw.pop("init_std")
+    m = vn.VerseNexLM(dtype="f32", **kw)
+    m.load_state_dict(sd)
+    toks = np.random.default_rng(1).integers(0, 50, (1, 50))
+    got = m.forward_cached(np.repeat(toks, 1400, 0), m.new_cache(1400, 6050), want_logits=False, want_hidden=True).numpy()
+    want, _ = OM.forward_hidden(sd, cfg, toks)
+    assert np.max(np.abs(got - want)) / np.max(np.abs(want)) < 1e-4

@@ -637,8 +637,8 @@ inline TrisparsePlan trisparse_plan(const vn_ctx* ctx, const AttnArgs& a, int B)
   TrisparsePlan p = plan(8);
   if (n_items <= 4 || 2 * p.blocks < 3 * sm || p.per_sm < 3) p = plan(4);
   const long long once = p.per_sm * sm;
-  p.rows = p.smem <= TR_SMEM && B <= 65535 && a.n_kv <= 65535 &&
-           (p.blocks <= once || p.per_sm >= 4 || (p.per_sm == 3 && (p.R == 8 || p.blocks <= 6 * once)));
+  const bool pays = p.blocks <= once || p.per_sm >= 4 || (p.per_sm == 3 && (p.R == 8 || p.blocks <= 6 * once));
+  p.rows = p.smem <= TR_SMEM && B <= 65535 && a.n_kv <= 65535 && (pays || (long long)B * a.Tn > 65535);   // the other kernel's grid ends there
   return p;
 }
 
