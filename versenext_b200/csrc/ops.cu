@@ -442,7 +442,6 @@ int32_t vn_attention(vn_ctx* ctx, const float* q, const float* k, const float* v
   VN_CHECK_CTX(ctx);
   VN_REQUIRE(ctx, q && k && v && out && BH >= 0 && Tq >= 0 && Tk >= 1 && D >= 1, "bad arguments");
   VN_REQUIRE(ctx, BH < 65536, "too many batch*heads");
-  VN_REQUIRE(ctx, Tq < (1ll << 31), "too many queries");
   if (BH * Tq == 0) return VN_OK;
   // one limit for every shape, whichever kernel takes it (the row kernel keeps a row of scores in shared memory, the tile kernel none)
   VN_REQUIRE(ctx, Tk <= AT_MAX_TK, "Tk %lld too long for the backend attention op", (long long)Tk);
@@ -463,6 +462,7 @@ int32_t vn_attention(vn_ctx* ctx, const float* q, const float* k, const float* v
     if (D <= 64) return launch_attention_tile<64>(ctx, q, k, v, mask, out, BH, Tq, Tk, (int)D, scale, vec);
     return launch_attention_tile<128>(ctx, q, k, v, mask, out, BH, Tq, Tk, (int)D, scale, vec);
   }
+  VN_REQUIRE(ctx, Tq < (1ll << 31), "too many queries");
   int lpk = 1;
   while (lpk < 32 && lpk * 4 < D) lpk *= 2;
   const size_t smem = attention_row_smem(Tk);
